@@ -755,6 +755,7 @@ struct BatchedSim {
             P.in_pay_mult = b.in->pay_mult;
             P.in_pay_shift = b.in->pay_shift;
             P.in_pay_stride = b.in->pay_stride;
+            P.in_index_bits = detail::index_bits(*std::max_element(cap.begin(), cap.end()));
             if (b.sort && shape.stage_bytes >= 1024u && stage_pays(*b.in)) {
                 P.stage_bytes = (shape.stage_bytes + 15u) & ~15u;
                 smem = P.stage_bytes + static_cast<unsigned int>(sizeof(StageHeader));

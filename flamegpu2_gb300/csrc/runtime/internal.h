@@ -38,6 +38,14 @@ struct SpatialRecordLayout {
 SpatialRecordLayout spatial_record_layout(const std::vector<std::pair<uint32_t, uint32_t>>& vars, int dims,
                                           const char* what);
 
+// Bits that hold every index below n (at least 1, at most 31): a search's range
+// words keep a first message in as many bits and its length in the others.
+inline uint32_t index_bits(uint64_t n) {
+    uint32_t bits = 1;
+    while (bits < 31u && (1ull << bits) < n) ++bits;
+    return bits;
+}
+
 // Whether a block's neighbourhood window (the sorted records from one z/y slab
 // below its lowest bin to one above its highest) is expected to fit a staging
 // buffer of stage_bytes, with per_bin messages in every bin of grid g. Staging

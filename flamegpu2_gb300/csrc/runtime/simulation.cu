@@ -1771,6 +1771,7 @@ struct SimulationImpl {
                 P.in_pay_mult = f.in->pay_mult;
                 P.in_pay_shift = f.in->pay_shift;
                 P.in_pay_stride = f.in->pay_stride;
+                P.in_index_bits = detail::index_bits(f.in->capacity);
                 P.in_pbm_alloc = f.in->pbm_alloc;
                 if (f.stage && cuda_config.message_stage_bytes >= 1024u &&
                     stage_window_fits(*f.in, cuda_config.message_stage_bytes, agent_block(grid_rows(l))))

@@ -163,6 +163,7 @@ struct LaunchParams {
     // record layout: location words first, then each other variable at byte
     // 4 * dims + slot * in_pay_stride, slot = table_slot(in_pay_mult, in_pay_shift, hash)
     uint32_t in_pay_mult, in_pay_shift, in_pay_stride;
+    uint32_t in_index_bits;      // bits that hold any of an instance's sorted message indices
     uint32_t in_pbm_alloc;       // PBM entries readable (multiple of 4, >= binCount + 1)
     uint32_t in_dims[3];         // array message input: dimensions (1 past the last used)
     uint32_t out_dims[3];        // array message output: dimensions

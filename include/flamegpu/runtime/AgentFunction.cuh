@@ -28,8 +28,6 @@ namespace detail {
 typedef cudaError_t (*AgentFunctionLauncher)(const LaunchParams& p, unsigned int grid, unsigned int block,
                                              unsigned int smem, cudaStream_t stream, bool pdl);
 
-constexpr unsigned int kAgentBlock = 128;
-
 #ifdef __CUDACC__
 // Instance of row `row` in a batched launch (instances ordered by row_begin).
 __device__ __forceinline__ uint32_t batch_find(const BatchInstanceRT* b, uint32_t n, uint32_t row) {
@@ -44,25 +42,12 @@ __device__ __forceinline__ uint32_t batch_find(const BatchInstanceRT* b, uint32_
     return lo;
 }
 
-// Fill the block's instance context for rows starting at `base`. Single
-// simulations take it from the launch; batched launches from the instance
-// owning `base` (instance segments start at multiples of kAgentBlock, so a
-// block never straddles two instances).
-__device__ __forceinline__ void fill_ctx(const LaunchParams& P, uint32_t base, uint32_t n_single) {
+// Fill the block's instance context for rows starting at `base` of a batched
+// launch, from the instance owning `base` (instance segments start at
+// multiples of kAgentBlock, so a block never straddles two instances).
+__device__ __forceinline__ void fill_ctx(const LaunchParams& P, uint32_t base) {
     if (threadIdx.x != 0) return;
     InstanceCtx& c = ctx();
-    if (!P.batch) {
-        c.grid = P.in_grid;
-        c.pbm = P.in_pbm;
-        c.pbm_alloc = P.in_pbm_alloc;
-        c.step = P.d_step ? *P.d_step : 0u;
-        c.env = P.env;
-        c.seed = P.seed;
-        c.row_begin = P.d_first ? *P.d_first : 0u;  // rows before it failed the function's condition
-        c.count = n_single;
-        c.inst = 0;
-        return;
-    }
     const uint32_t k = batch_find(P.batch, P.batch_n, base);
     const BatchInstanceRT& I = P.batch[k];
     c.grid = I.in_grid;
@@ -88,16 +73,19 @@ __device__ __forceinline__ void fill_ctx(const LaunchParams& P, uint32_t base, u
 #define FLAMEGPU_AGENT_MIN_BLOCKS 8
 #endif
 
-template <typename F, int MINB>
+// BATCH: a batched launch (P.batch); STAGE: blocks stage their neighbourhood
+// windows (P.stage_bytes, spatial input only).
+template <typename F, int MINB, bool BATCH, bool STAGE>
 __global__ void __launch_bounds__(kAgentBlock, MINB) agent_function_kernel(const __grid_constant__ LaunchParams P) {
     grid_dependency_enter();
+    const Launch L{P, BATCH, STAGE};
     using MsgIn = typename F::MessageIn;
     using MsgOut = typename F::MessageOut;
     // rows to visit: the population (single) or every row of the batch
-    const uint32_t n = P.batch ? P.max_n : (P.d_n ? min(*P.d_n, P.max_n) : P.max_n);
-    const uint32_t first_row = (!P.batch && P.d_first) ? min(*P.d_first, n) : 0u;
+    const uint32_t n = BATCH ? P.max_n : (P.d_n ? min(*P.d_n, P.max_n) : P.max_n);
+    const uint32_t first_row = (!BATCH && P.d_first) ? min(*P.d_first, n) : 0u;
     // message rows: after those already output to the list this step (append), else from 0
-    const uint32_t msg_base = (!P.batch && P.msg_out_base) ? *P.msg_out_base : 0u;
+    const uint32_t msg_base = (!BATCH && P.msg_out_base) ? *P.msg_out_base : 0u;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         // a launch over no agents leaves the list as it was (the reference skips
         // such a function, CUDASimulation.cu:1050-1059): a persistent list keeps
@@ -113,23 +101,17 @@ __global__ void __launch_bounds__(kAgentBlock, MINB) agent_function_kernel(const
     bool first = true;
     uint32_t out_of_order = 0u;  // keyed targets whose rows were not in key order
     uint32_t alive_rows = 0u;    // rows this thread left ALIVE (survivor count for the compaction)
-    if (!P.batch) {
-        fill_ctx(P, 0, n);
-        __syncthreads();
-    }
     for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
-        if (P.batch) {
+        if constexpr (BATCH) {
             __syncthreads();  // the previous round is done with the context
-            fill_ctx(P, base, 0);
+            fill_ctx(P, base);
             __syncthreads();
         }
         const uint32_t idx = base + threadIdx.x;
         // rows past the instance's count are padding (batched) / past the population (single)
-        const uint32_t limit = P.batch ? ctx().row_begin + ctx().count : n;
+        const uint32_t limit = BATCH ? ctx().row_begin + ctx().count : n;
         const uint32_t live = idx < limit ? idx : 0xFFFFFFFFu;
-        if constexpr (kDims != 0) {
-            if (P.stage_bytes) stage_window<kDims>(P, idx, live != 0xFFFFFFFFu, first);
-        }
+        if constexpr (STAGE) stage_window<kDims>(L, idx, live != 0xFFFFFFFFu, first);
         first = false;
         if (live == 0xFFFFFFFFu) continue;
         if (idx < first_row) {  // failed the condition: kept as it is
@@ -149,7 +131,7 @@ __global__ void __launch_bounds__(kAgentBlock, MINB) agent_function_kernel(const
             if (P.keyed[1].dims == 3) pre[2] = P.keyed[1].z[idx];
             pre_key = key_target_key(P.keyed[1], true, pre[0], pre[1], pre[2]);
         }
-        DeviceAPI<MsgIn, MsgOut> api(P, idx, msg_row);
+        DeviceAPI<MsgIn, MsgOut> api(L, idx, msg_row);
         const AGENT_STATUS st = F()(&api);
         alive_rows += st == ALIVE ? 1u : 0u;
         if (P.death_flags) {
@@ -202,12 +184,11 @@ template <typename C>
 __global__ void __launch_bounds__(kAgentBlock) agent_condition_kernel(const __grid_constant__ LaunchParams P) {
     grid_dependency_enter();
     const uint32_t n = P.d_n ? min(*P.d_n, P.max_n) : P.max_n;
-    fill_ctx(P, 0, n);
-    __syncthreads();
+    const Launch L{P, false, false};
     for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx <= P.max_n; idx += gridDim.x * blockDim.x) {
         uint32_t fail = 0u;
         if (idx < n) {
-            ReadOnlyDeviceAPI api(P, idx);
+            ReadOnlyDeviceAPI api(L, idx);
             fail = C()(&api) ? 0u : 1u;
         }
         P.cond_fail[idx] = fail;
@@ -220,17 +201,17 @@ cudaError_t launch_agent_condition(const LaunchParams& p, unsigned int grid, uns
     return launch_kernel(pdl, agent_condition_kernel<C>, grid, block, 0, stream, p);
 }
 
-template <typename F, int MINB>
+template <typename F, int MINB, bool BATCH, bool STAGE>
 cudaError_t launch_agent_variant(const LaunchParams& p, unsigned int grid, unsigned int block, unsigned int smem,
                                  cudaStream_t stream, bool pdl) {
     static unsigned int configured = 48u * 1024u;
     if (smem > configured) {
-        const cudaError_t e = cudaFuncSetAttribute(agent_function_kernel<F, MINB>,
+        const cudaError_t e = cudaFuncSetAttribute(agent_function_kernel<F, MINB, BATCH, STAGE>,
                                                    cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
         if (e != cudaSuccess) return e;
         configured = smem;
     }
-    return launch_kernel(pdl, agent_function_kernel<F, MINB>, grid, block, smem, stream, p);
+    return launch_kernel(pdl, agent_function_kernel<F, MINB, BATCH, STAGE>, grid, block, smem, stream, p);
 }
 
 inline unsigned int device_sm_count() {
@@ -245,13 +226,22 @@ inline unsigned int device_sm_count() {
 
 // block: 32, 64 or 128 threads (kAgentBlock divides into whole blocks). A
 // launch of at most one 128-thread block's worth of threads per SM takes the
-// variant compiled without a register cap: its blocks fit the SMs anyway.
+// variant compiled without a register cap: its blocks fit the SMs anyway. So
+// does a launch that stages windows: their shared memory holds it to a few
+// blocks per SM.
 template <typename F>
 cudaError_t launch_agent_function(const LaunchParams& p, unsigned int grid, unsigned int block, unsigned int smem,
                                   cudaStream_t stream, bool pdl) {
+    using MsgIn = typename F::MessageIn;
+    constexpr bool kSpatial = std::is_same<MsgIn, MessageSpatial3D>::value || std::is_same<MsgIn, MessageSpatial2D>::value;
+    if constexpr (kSpatial) {
+        if (p.stage_bytes) return p.batch ? launch_agent_variant<F, 1, true, true>(p, grid, block, smem, stream, pdl)
+                                          : launch_agent_variant<F, 1, false, true>(p, grid, block, smem, stream, pdl);
+    }
+    if (p.batch) return launch_agent_variant<F, FLAMEGPU_AGENT_MIN_BLOCKS, true, false>(p, grid, block, smem, stream, pdl);
     if (static_cast<uint64_t>(grid) * block <= static_cast<uint64_t>(device_sm_count()) * kAgentBlock)
-        return launch_agent_variant<F, 1>(p, grid, block, smem, stream, pdl);
-    return launch_agent_variant<F, FLAMEGPU_AGENT_MIN_BLOCKS>(p, grid, block, smem, stream, pdl);
+        return launch_agent_variant<F, 1, false, false>(p, grid, block, smem, stream, pdl);
+    return launch_agent_variant<F, FLAMEGPU_AGENT_MIN_BLOCKS, false, false>(p, grid, block, smem, stream, pdl);
 }
 #endif
 

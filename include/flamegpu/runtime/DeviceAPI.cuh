@@ -42,11 +42,39 @@ __device__ __forceinline__ void device_error(const LaunchParams& P, uint32_t cod
     }
 }
 
-// The calling block's instance context (shared memory).
+// Threads of the largest agent-function block.
+constexpr unsigned int kAgentBlock = 128;
+
+// The calling block's instance context (shared memory; batched launches only).
 __device__ __forceinline__ InstanceCtx& ctx() {
     __shared__ InstanceCtx c;
     return c;
 }
+
+/** A launch as its agents' code sees it: the parameters, and which of the
+ * kernel's variants runs. `batch` and `stage` are literals of the variant, so
+ * once inlined every choice below folds away: a single simulation reads its
+ * grid, PBM and environment straight from the parameter space (no context in
+ * shared memory, no barrier before the first agent), and a launch without a
+ * staged window reads records as global memory through 64-bit arithmetic on
+ * launch constants. */
+struct Launch {
+    const LaunchParams& P;
+    bool batch;  // ctx() holds the instance of the block's rows
+    bool stage;  // the block may have a staged window
+    __device__ __forceinline__ operator const LaunchParams&() const { return P; }
+    __device__ __forceinline__ const fg_spatial_grid& grid() const { return batch ? ctx().grid : P.in_grid; }
+    __device__ __forceinline__ const uint32_t* pbm() const { return batch ? ctx().pbm : P.in_pbm; }
+    __device__ __forceinline__ uint32_t pbm_alloc() const { return batch ? ctx().pbm_alloc : P.in_pbm_alloc; }
+    __device__ __forceinline__ uint32_t step() const { return batch ? ctx().step : (P.d_step ? *P.d_step : 0u); }
+    __device__ __forceinline__ const char* env() const { return batch ? ctx().env : P.env; }
+    __device__ __forceinline__ uint64_t seed() const { return batch ? ctx().seed : P.seed; }
+    // first row of the instance; in a single simulation, the rows before it failed the function's condition
+    __device__ __forceinline__ uint32_t row_begin() const { return batch ? ctx().row_begin : (P.d_first ? *P.d_first : 0u); }
+    // first row of the instance's sorted messages
+    __device__ __forceinline__ uint32_t row_base() const { return batch ? ctx().row_begin : 0u; }
+    __device__ __forceinline__ uint32_t inst() const { return batch ? ctx().inst : 0u; }
+};
 
 // Address of element `elem` of variable `hash` in row `row` of table `t`.
 // Returns null (after recording a device error) when seatbelts are on and the
@@ -152,32 +180,11 @@ __device__ __forceinline__ const char* stage_records(const StageHeader* h) {
     return dyn_smem() + sizeof(StageHeader) + static_cast<size_t>(h->pbm_n) * 4u;
 }
 
-// PBM entry h of the input message list: from the staged slice when inside it.
-__device__ __forceinline__ uint32_t pbm_at(const LaunchParams& P, uint32_t h) {
-    if (P.stage_bytes) {
-        const StageHeader* s = stage_hdr();
-        const uint32_t r = h - s->pbm_lo;
-        if (r < s->pbm_n) return stage_pbm()[r];
-    }
-    return __ldg(ctx().pbm + h);
-}
-
-// Read of a variable of message `index` of the input list: staged copy when
-// the message is inside the block's window, else the sorted records in HBM.
+// Read of a variable of message `index` of an input list of columns.
 template <typename T>
 __device__ __forceinline__ T read_msg(const LaunchParams& P, uint32_t hash, uint32_t index, uint32_t elem) {
     const T* a = var_addr<T>(P, &P.T.msg_in, hash, index, elem);
-    if (!a) return T{};
-    if (P.stage_bytes) {
-        const StageHeader* s = stage_hdr();
-        const uint32_t r = index - s->rec_lo;
-        if (r < s->rec_n) {
-            const size_t row = static_cast<size_t>(index) * P.in_record_bytes;
-            const size_t off = static_cast<size_t>(reinterpret_cast<const char*>(a) - P.in_records) - row;
-            return *reinterpret_cast<const T*>(stage_records(s) + static_cast<size_t>(r) * P.in_record_bytes + off);
-        }
-    }
-    return ldg_any(a);
+    return a ? ldg_any(a) : T{};
 }
 
 // Byte offset of element `elem` of variable `hash` inside a sorted message
@@ -229,7 +236,8 @@ __device__ __forceinline__ bool stage_wait(StageHeader* h, uint32_t phase) {
 // a contiguous range of the sorted records, copied with TMA bulk copies
 // (cp.async.bulk) completing on an mbarrier. All threads of the block call it.
 template <int DIMS>
-__device__ void stage_window(const LaunchParams& P, uint32_t idx, bool active, bool first) {
+__device__ void stage_window(const Launch& L, uint32_t idx, bool active, bool first) {
+    const LaunchParams& P = L.P;
     __shared__ uint32_t s_min, s_max;
     StageHeader* h = stage_hdr();
     if (threadIdx.x == 0) {
@@ -244,7 +252,7 @@ __device__ void stage_window(const LaunchParams& P, uint32_t idx, bool active, b
     }
     uint32_t key = 0xFFFFFFFFu, kmax = 0u;
     if (active) {
-        const fg_spatial_grid& g = ctx().grid;
+        const fg_spatial_grid& g = L.grid();
         const float x = read_rw<float>(P, &P.T.agent, VarName("x").hash, idx);
         const float y = read_rw<float>(P, &P.T.agent, VarName("y").hash, idx);
         const float z = DIMS == 3 ? read_rw<float>(P, &P.T.agent, VarName("z").hash, idx) : 0.0f;
@@ -272,15 +280,15 @@ __device__ void stage_window(const LaunchParams& P, uint32_t idx, bool active, b
         // after a wait that gave up, copies of that window may still land on
         // the mbarrier and in the buffer: the block reads from HBM from then on
         if (s_min != 0xFFFFFFFFu && !h->off) {
-            const fg_spatial_grid& g = ctx().grid;
-            const uint32_t* pbm = ctx().pbm;
+            const fg_spatial_grid& g = L.grid();
+            const uint32_t* pbm = L.pbm();
             const uint32_t B = g.binCount;
             const uint32_t span = DIMS == 3 ? g.gridDim[0] * g.gridDim[1] + g.gridDim[0] + 1u : g.gridDim[0] + 1u;
             const uint32_t hlo = s_min > span ? s_min - span : 0u;
             const uint32_t hhi = (s_max + span < B) ? s_max + span : B - 1u;
             const uint32_t plo = hlo & ~3u;
             uint32_t pend = (hhi + 2u + 3u) & ~3u;
-            if (pend > ctx().pbm_alloc) pend = ctx().pbm_alloc;
+            if (pend > L.pbm_alloc()) pend = L.pbm_alloc();
             const uint32_t pn = pend - plo;
             const uint32_t rlo = __ldg(pbm + hlo), rhi = __ldg(pbm + hhi + 1u);
             const size_t pbytes = static_cast<size_t>(pn) * 4u;
@@ -811,6 +819,36 @@ class MessageBucket {
     };
 };
 
+/** The staged window of the calling block, cached in registers by a filter. */
+struct Window {
+    uint32_t rec_lo = 0, rec_n = 0, pbm_lo = 0, pbm_n = 0;
+    const char* rec = nullptr;
+    const uint32_t* pbm = nullptr;
+    const uint32_t* gpbm = nullptr;  // the instance's PBM in HBM
+    __device__ explicit Window(const detail::Launch& L) {
+        gpbm = L.pbm();
+        if (!L.stage) return;
+        const detail::StageHeader* h = detail::stage_hdr();
+        rec_lo = h->rec_lo;
+        rec_n = h->rec_n;
+        pbm_lo = h->pbm_lo;
+        pbm_n = h->pbm_n;
+        pbm = detail::stage_pbm();
+        rec = detail::stage_records(h);
+    }
+    __device__ uint32_t pbm_at(const detail::Launch& L, uint32_t h) const {
+        if (!L.stage) return __ldg(gpbm + h);
+        const uint32_t r = h - pbm_lo;
+        return r < pbm_n ? pbm[r] : __ldg(gpbm + h);
+    }
+    __device__ const char* row(const detail::Launch& L, uint32_t index) const {
+        const char* g = L.P.in_records + static_cast<size_t>(index) * L.P.in_record_bytes;
+        if (!L.stage) return g;
+        const uint32_t r = index - rec_lo;
+        return r < rec_n ? rec + static_cast<size_t>(r) * L.P.in_record_bytes : g;
+    }
+};
+
 /**
  * A message of a spatial input list: a view of its sorted record. `row` is
  * the record's address — in the block's shared-memory window when the
@@ -867,274 +905,289 @@ class RecordView {
     const char* row;
 };
 
-/**
- * Spatially partitioned messages; the iterators visit the reference's
- * Moore neighbourhood in the reference's order. DIMS = 2 or 3.
- * Filter: 3^(DIMS-1) x-strips, y-offset outer, z-offset inner, each strip
- * PBM[hash(x-1)] .. PBM[hash(x+1)+1] with x clamped (MessageSpatial3DDevice.cuh:693-719).
- * WrapFilter: 3^DIMS single bins, x offset outer, then y, z offset inner
- * (nextCell, MessageSpatial3DDevice.cuh:264-276), every axis taken modulo
- * gridDim (:727-749); no radius test — user code filters.
- * Both iterators first read the PBM bounds of all their strips or cells in
- * lock step (unrolled, so every hash is a sum of registers) and keep one bit
- * per non-empty one; they then visit only those, in order, loading the next
- * one's bounds while the current one is being read. A lane whose strip or
- * cell ends thus moves to the next non-empty one in one step, so the lanes of
- * a warp advance at most once per message visited instead of each stepping
- * through empty cells on its own (in sparse neighbourhoods most are empty).
- * A cell lies wholly inside or wholly outside the block's staged window, so
- * within a cell the record address just advances by one record.
+/*
+ * Spatially partitioned messages; the iterators visit the reference's Moore
+ * neighbourhood in the reference's order, with no radius test (user code
+ * filters). A clamped search visits 3^(DIMS-1) x-strips, y-offset outer,
+ * z-offset inner, each strip PBM[hash(x-1)] .. PBM[hash(x+1)+1] with x
+ * clamped; a wrapped one 3^DIMS single bins, x offset outer, then y, z offset
+ * inner, every axis taken modulo gridDim.
+ *
+ * What bounds it: in sparse neighbourhoods the lanes of a warp change range at
+ * different messages, so nearly every message a warp visits pays for a change;
+ * in dense ones the issue slots (the user's own arithmetic). So the cost of
+ * entering the next range is what the cursors below keep small:
+ *  - the wrapped search's 27 (9) bins: their bounds are read once and kept in
+ *    shared memory, one word each. Recomputing the hash with its three wrapped
+ *    axes and reading the bounds again took 7,000 warp instructions a warp and
+ *    260 us for the Boids iterate of 1,048,576 agents, against 4,860 and 197
+ *    us; the same words in local memory 278 us (their lines cost the records
+ *    their place in L1, hit rate 84 -> 72%);
+ *  - the clamped search's 9 (3) strips: the hash is two multiply-adds from the
+ *    corner strip, so the strips are a bit mask and the bounds are read again.
+ *    100,003 Boids: 37.3 -> 33.4 us. Words in shared memory as above would
+ *    give 31.3 us there, but take 84 KB of L1 from the 12 resident blocks of
+ *    the 8,388,608-agent Gaussian mixture, 371 -> 377 ms against 366 ms.
+ * A range lies wholly inside or wholly outside the block's staged window, so
+ * within a range the record address just advances by one record.
  */
-__device__ __forceinline__ uint32_t pick(int r, uint32_t a, uint32_t b, uint32_t c) {
-    return r == 0 ? a : (r == 1 ? b : c);
-}
 
-/** The staged window of the calling block, cached in registers by a filter. */
-struct Window {
-    uint32_t rec_lo = 0, rec_n = 0, pbm_lo = 0, pbm_n = 0;
-    const char* rec = nullptr;
-    const uint32_t* pbm = nullptr;
-    const uint32_t* gpbm = nullptr;  // the instance's PBM in HBM
-    __device__ void load(const detail::LaunchParams& P) {
-        gpbm = detail::ctx().pbm;
-        if (!P.stage_bytes) return;
-        const detail::StageHeader* h = detail::stage_hdr();
-        rec_lo = h->rec_lo;
-        rec_n = h->rec_n;
-        pbm_lo = h->pbm_lo;
-        pbm_n = h->pbm_n;
-        pbm = detail::stage_pbm();
-        rec = detail::stage_records(h);
+/** The x strips of a clamped search (MessageSpatial3DDevice.cuh:693-719), the
+ * non-empty ones in visit order. One bit per strip not yet entered; the next
+ * one's bounds are read while the current one is walked. */
+template <int DIMS>
+class StripCursor {
+    static constexpr int kStrips = DIMS == 3 ? 9 : 3;
+
+ public:
+    // a search keeps nothing but its origin: every walk reads the bounds itself
+    struct Shared {
+        __device__ __forceinline__ Shared(const detail::Launch&, const Window&, bool&, const float (&)[3]) {}
+    };
+    __device__ __forceinline__ StripCursor(const detail::Launch& l, const Window& w, const Shared&, const float (&p)[3])
+        : L(l), win(w) {
+        const fg_spatial_grid& g = L.grid();
+        const int dx = static_cast<int>(g.gridDim[0]), dy = static_cast<int>(g.gridDim[1]), dz = static_cast<int>(g.gridDim[2]);
+        const int cx = detail::grid_cell(g, 0, p[0]), cy = detail::grid_cell(g, 1, p[1]);
+        const int cz = DIMS == 3 ? detail::grid_cell(g, 2, p[2]) : 0;
+        const int x0 = cx > 0 ? cx - 1 : 0;
+        width = static_cast<uint32_t>((cx + 1 < dx ? cx + 1 : dx - 1) - x0 + 1);
+        // the first strip's first cell; outside the grid its hash wraps, and no bit selects it
+        corner = static_cast<uint32_t>(x0 + (cy - 1) * dx + (DIMS == 3 ? (cz - 1) * dx * dy : 0));
+#pragma unroll
+        for (int t = 0; t < kStrips; ++t) {
+            const int ay = cy + (DIMS == 3 ? t / 3 : t) - 1, az = cz + (DIMS == 3 ? t % 3 - 1 : 0);
+            const bool inside = ay >= 0 && ay < dy && (DIMS == 2 || (az >= 0 && az < dz));
+            if (inside) {
+                const uint32_t h = hash(t);
+                todo |= (win.pbm_at(L, h) < win.pbm_at(L, h + width) ? 1u : 0u) << t;
+            }
+        }
+        read_ahead();
     }
-    __device__ uint32_t pbm_at(const detail::LaunchParams& P, uint32_t h) const {
-        const uint32_t r = h - pbm_lo;
-        return r < pbm_n ? pbm[r] : __ldg(gpbm + h);
+    __device__ __forceinline__ void next(uint32_t& b, uint32_t& e) {
+        b = nb;
+        e = ne;
+        read_ahead();
     }
-    __device__ const char* row(const detail::LaunchParams& P, uint32_t index) const {
-        const uint32_t r = index - rec_lo;
-        return r < rec_n ? rec + static_cast<size_t>(r) * P.in_record_bytes
-                         : P.in_records + static_cast<size_t>(index) * P.in_record_bytes;
+
+ private:
+    __device__ __forceinline__ uint32_t hash(uint32_t t) const {
+        const fg_spatial_grid& g = L.grid();
+        if (DIMS == 2) return corner + t * g.gridDim[0];
+        const uint32_t q = (t * 11u) >> 5;  // t / 3, t < 9
+        return corner + q * g.gridDim[0] + (t - 3u * q) * (g.gridDim[0] * g.gridDim[1]);
     }
+    // an empty range when none is left
+    __device__ __forceinline__ void read_ahead() {
+        nb = ne = 0;
+        if (todo) {
+            const uint32_t h = hash(static_cast<uint32_t>(__ffs(todo) - 1));
+            todo &= todo - 1u;
+            nb = win.pbm_at(L, h);
+            ne = win.pbm_at(L, h + width);
+        }
+    }
+    const detail::Launch L;
+    const Window win;
+    uint32_t corner, width;  // strip t: cells hash(t) .. hash(t) + width - 1
+    uint32_t todo = 0, nb, ne;
+};
+
+/** The single bins of a wrapped search (MessageSpatial3DDevice.cuh:264-276,
+ * :727-749), the non-empty ones in visit order. Their bounds are read once,
+ * when the search is made, and kept as one word each in shared memory (one
+ * column per thread): the first message below, the length above bit
+ * `in_index_bits`, then an end word; entering the next bin is one shared
+ * load, issued one bin ahead. Where a length does not fit, or while another
+ * search of the same thread (a nested loop) has its words there, or for a
+ * copied search, the walk steps through the bins instead. */
+template <int DIMS>
+class CellCursor {
+    static constexpr int kCells = DIMS == 3 ? 27 : 9;
+    // hash terms of the offsets -1, 0, +1 on each axis, modulo gridDim
+    // (MessageSpatial3DDevice.cuh:736-738)
+    struct Terms {
+        uint32_t hx[3], hy[3], hz[3];
+        __device__ __forceinline__ Terms(const detail::Launch& L, const float (&p)[3]) {
+            const fg_spatial_grid& g = L.grid();
+            axis(hx, detail::grid_cell(g, 0, p[0]), g.gridDim[0], 1u);
+            axis(hy, detail::grid_cell(g, 1, p[1]), g.gridDim[1], g.gridDim[0]);
+            if (DIMS == 3) axis(hz, detail::grid_cell(g, 2, p[2]), g.gridDim[2], g.gridDim[0] * g.gridDim[1]);
+        }
+        __device__ __forceinline__ uint32_t hash(int t) const {
+            return DIMS == 3 ? pick(hx, t / 9) + pick(hy, (t / 3) % 3) + pick(hz, t % 3) : pick(hx, t / 3) + pick(hy, t % 3);
+        }
+        static __device__ __forceinline__ uint32_t pick(const uint32_t (&h)[3], int r) {
+            return r == 0 ? h[0] : (r == 1 ? h[1] : h[2]);
+        }
+        // cell c is in [0, d), so c - 1 and c + 1 need at most one turn
+        static __device__ __forceinline__ void axis(uint32_t (&h)[3], int c, uint32_t d, uint32_t scale) {
+            const uint32_t u = static_cast<uint32_t>(c);
+            h[0] = (u == 0u ? d - 1u : u - 1u) * scale;
+            h[1] = u * scale;
+            h[2] = (u + 1u == d ? 0u : u + 1u) * scale;
+        }
+    };
+    static __device__ __forceinline__ uint32_t* column() {
+        __shared__ uint32_t words[(kCells + 2) * detail::kAgentBlock];
+        return words + threadIdx.x;
+    }
+
+ public:
+    // holds the thread's words while it lives
+    struct Shared {
+        bool& busy;
+        const bool owner;
+        bool listed = false;
+        __device__ __forceinline__ Shared(const detail::Launch& L, const Window& win, bool& in_use, const float (&p)[3])
+            : busy(in_use), owner(!in_use) {
+            if (!owner) return;
+            busy = true;
+            const Terms terms(L, p);
+            uint32_t* w = column();
+            const uint32_t bits = L.P.in_index_bits, base = L.row_base();
+            listed = true;
+#pragma unroll
+            for (int t = 0; t < kCells; ++t) {
+                const uint32_t h = terms.hash(t);
+                const uint32_t b = win.pbm_at(L, h), e = win.pbm_at(L, h + 1u);
+                const uint32_t len = b < e ? e - b : 0u;  // a PBM whose scan gave up may run backwards
+                *w = (b - base) | (len << bits);
+                w += len ? detail::kAgentBlock : 0u;
+                listed = listed && (len >> 1) >> (31u - bits) == 0u;
+            }
+            w[0] = w[detail::kAgentBlock] = 0u;
+        }
+        __device__ __forceinline__ Shared(const Shared& o) : busy(o.busy), owner(false) {}
+        __device__ __forceinline__ ~Shared() {
+            if (owner) busy = false;
+        }
+    };
+    __device__ __forceinline__ CellCursor(const detail::Launch& l, const Window& w, const Shared& s, const float (&p)[3])
+        : L(l), win(w), listed(s.listed), at(column()), loc{p[0], p[1], p[2]} {
+        if (listed) ahead = *at;
+    }
+    __device__ __forceinline__ void next(uint32_t& b, uint32_t& e) {
+        if (listed) {
+            const uint32_t bits = L.P.in_index_bits;
+            b = L.row_base() + (ahead & ((1u << bits) - 1u));
+            e = b + (ahead >> bits);
+            at += detail::kAgentBlock;
+            ahead = *at;  // in flight while this bin is read
+            return;
+        }
+        const Terms terms(L, loc);
+        b = e = 0;
+        while (!(b < e) && t < kCells) {
+            const uint32_t h = terms.hash(t++);
+            b = win.pbm_at(L, h);
+            e = win.pbm_at(L, h + 1u);
+        }
+    }
+
+ private:
+    const detail::Launch L;
+    const Window win;
+    const bool listed;
+    const uint32_t* at;  // the word read ahead
+    uint32_t ahead = 0;
+    int t = 0;           // next bin, when not listed
+    const float loc[3];
+};
+
+/** A search's messages: the ranges its cursor gives, one after another. */
+template <typename Cursor, typename MessageT>
+class Search {
+ public:
+    class iterator {
+     public:
+        __device__ __forceinline__ iterator(const Search& s, bool at_end)
+            : L(s.L), win(s.win), cursor(s.L, s.win, s.shared, s.loc), m(s.L, s.loc), end_(0) {
+            if (!at_end) advance();
+        }
+        __device__ __forceinline__ iterator& operator++() {
+            m.row += L.P.in_record_bytes;
+            if (++m.index >= end_) advance();
+            return *this;
+        }
+        __device__ __forceinline__ bool operator!=(const iterator&) const { return m.index < end_; }
+        __device__ __forceinline__ bool operator==(const iterator& o) const { return !(*this != o); }
+        __device__ __forceinline__ const MessageT& operator*() const { return m; }
+        __device__ __forceinline__ const MessageT* operator->() const { return &m; }
+
+     private:
+        // enter the next range (past the last: an empty one, which ends the loop)
+        __device__ __forceinline__ void advance() {
+            cursor.next(m.index, end_);
+            m.row = win.row(L, m.index);
+        }
+        const detail::Launch L;
+        const Window win;
+        Cursor cursor;
+        MessageT m;
+        uint32_t end_;
+    };
+
+    __device__ __forceinline__ Search(const detail::Launch& l, bool& in_use, float x, float y, float z)
+        : L(l), win(l), loc{x, y, z}, shared(l, win, in_use, loc) {}
+    __device__ __forceinline__ iterator begin() const { return iterator(*this, false); }
+    __device__ __forceinline__ iterator end() const { return iterator(*this, true); }
+
+ private:
+    const detail::Launch L;
+    const Window win;
+    const float loc[3];
+    const typename Cursor::Shared shared;
 };
 
 template <int DIMS>
 class SpatialIn {
  public:
-    static constexpr int kStrips = DIMS == 3 ? 9 : 3;
-    static constexpr int kCells = DIMS == 3 ? 27 : 9;
-
-    class Filter {
+    class ClampMessage : public RecordView<DIMS> {
      public:
-        class Message : public RecordView<DIMS> {
-         public:
-            __device__ Message(const detail::LaunchParams& p, uint32_t i) : RecordView<DIMS>(p, i) {}
-        };
-        class iterator {
-         public:
-            __device__ iterator(const Filter& f, bool at_end) : F(f), m(f.P, 0), end_(0) {
-                if (at_end) return;
-#pragma unroll
-                for (int t = 0; t < kStrips; ++t) {
-                    uint32_t b, e;
-                    bounds(t, b, e);
-                    todo_ |= (b < e ? 1u : 0u) << t;
-                }
-                prefetch();
-                advance();
-            }
-            __device__ iterator& operator++() {
-                m.row += F.P.in_record_bytes;
-                if (++m.index >= end_) advance();
-                return *this;
-            }
-            __device__ bool operator!=(const iterator&) const { return m.index < end_; }
-            __device__ bool operator==(const iterator& o) const { return !(*this != o); }
-            __device__ const Message& operator*() const { return m; }
-            __device__ const Message* operator->() const { return &m; }
-
-         private:
-            // PBM bounds of strip t (empty when the strip lies outside the grid)
-            __device__ void bounds(int t, uint32_t& b, uint32_t& e) const {
-                b = e = 0;
-                const int ry = DIMS == 3 ? t / 3 - 1 : t - 1;
-                const int rz = DIMS == 3 ? t % 3 - 1 : 0;
-                const int ay = F.cell[1] + ry, az = F.cell[2] + rz;
-                const fg_spatial_grid& g = detail::ctx().grid;
-                if (ay < 0 || ay >= static_cast<int>(g.gridDim[1])) return;
-                if (DIMS == 3 && (az < 0 || az >= static_cast<int>(g.gridDim[2]))) return;
-                const uint32_t h0 = detail::grid_hash(g, F.cell[0] - 1, ay, az);
-                const uint32_t h1 = detail::grid_hash(g, F.cell[0] + 1, ay, az);
-                b = F.win.pbm_at(F.P, h0);
-                e = F.win.pbm_at(F.P, h1 + 1);
-            }
-            // bounds of the next non-empty strip (an empty pair when none is left)
-            __device__ void prefetch() {
-                nb_ = ne_ = 0;
-                if (todo_) {
-                    const int t = __ffs(todo_) - 1;
-                    todo_ &= todo_ - 1u;
-                    bounds(t, nb_, ne_);
-                }
-            }
-            // enter the prefetched strip (index == end ends the loop)
-            __device__ void advance() {
-                m.index = nb_;
-                m.row = F.win.row(F.P, nb_);
-                end_ = ne_;
-                prefetch();  // in flight while this strip is read
-            }
-            const Filter& F;
-            Message m;
-            uint32_t end_;
-            uint32_t todo_ = 0;         // non-empty strips not yet entered
-            uint32_t nb_ = 0, ne_ = 0;  // bounds of the next one
-        };
-        __device__ Filter(const detail::LaunchParams& p, float x, float y, float z) : P(p) {
-            loc[0] = x;
-            loc[1] = y;
-            loc[2] = z;
-            const fg_spatial_grid& gc = detail::ctx().grid;
-            cell[0] = detail::grid_cell(gc, 0, x);
-            cell[1] = detail::grid_cell(gc, 1, y);
-            cell[2] = DIMS == 3 ? detail::grid_cell(gc, 2, z) : 0;
-            win.load(p);
+        __device__ __forceinline__ ClampMessage(const detail::Launch& l, const float (&)[3]) : RecordView<DIMS>(l.P, 0) {}
+    };
+    class WrapMessage : public RecordView<DIMS> {
+     public:
+        __device__ __forceinline__ WrapMessage(const detail::Launch& l, const float (&p)[3])
+            : RecordView<DIMS>(l.P, 0), L(l), x0(p[0]), y0(p[1]), z0(p[2]) {}
+        __device__ float getVirtualX() const { return getVirtualX(x0); }
+        __device__ float getVirtualY() const { return getVirtualY(y0); }
+        __device__ float getVirtualZ() const { return getVirtualZ(z0); }
+        __device__ float getVirtualX(float x1) const {
+            return detail::virtual_coord(x1, this->template getVariable<float>("x"), L.grid().width[0]);
         }
-        __device__ iterator begin() const { return iterator(*this, false); }
-        __device__ iterator end() const { return iterator(*this, true); }
+        __device__ float getVirtualY(float y1) const {
+            return detail::virtual_coord(y1, this->template getVariable<float>("y"), L.grid().width[1]);
+        }
+        __device__ float getVirtualZ(float z1) const {
+            return detail::virtual_coord(z1, this->template getVariable<float>("z"), L.grid().width[2]);
+        }
 
-        const detail::LaunchParams& P;
-        float loc[3];
-        int cell[3];
-        Window win;
+     private:
+        const detail::Launch L;
+        float x0, y0, z0;  // the search origin
+    };
+    class Filter : public Search<StripCursor<DIMS>, ClampMessage> {
+     public:
+        using Message = ClampMessage;
+        using Search<StripCursor<DIMS>, ClampMessage>::Search;
+    };
+    class WrapFilter : public Search<CellCursor<DIMS>, WrapMessage> {
+     public:
+        using Message = WrapMessage;
+        using Search<CellCursor<DIMS>, WrapMessage>::Search;
     };
 
-    class WrapFilter {
-     public:
-        class Message : public RecordView<DIMS> {
-         public:
-            __device__ Message(const detail::LaunchParams& p, uint32_t i, const WrapFilter* f)
-                : RecordView<DIMS>(p, i), F(f) {}
-            __device__ float getVirtualX() const { return getVirtualX(F->loc[0]); }
-            __device__ float getVirtualY() const { return getVirtualY(F->loc[1]); }
-            __device__ float getVirtualZ() const { return getVirtualZ(F->loc[2]); }
-            __device__ float getVirtualX(float x1) const {
-                return detail::virtual_coord(x1, this->template getVariable<float>("x"),
-                                             detail::ctx().grid.width[0]);
-            }
-            __device__ float getVirtualY(float y1) const {
-                return detail::virtual_coord(y1, this->template getVariable<float>("y"),
-                                             detail::ctx().grid.width[1]);
-            }
-            __device__ float getVirtualZ(float z1) const {
-                return detail::virtual_coord(z1, this->template getVariable<float>("z"),
-                                             detail::ctx().grid.width[2]);
-            }
-
-         private:
-            const WrapFilter* F;
-        };
-        class iterator {
-         public:
-            __device__ iterator(const WrapFilter& f, bool at_end) : F(f), m(f.P, 0, &f), end_(0) {
-                if (at_end) return;
-#pragma unroll
-                for (int t = 0; t < kCells; ++t) {
-                    const uint32_t h = hash(t);
-                    todo_ |= (F.win.pbm_at(F.P, h) < F.win.pbm_at(F.P, h + 1) ? 1u : 0u) << t;
-                }
-                prefetch();
-                advance();
-            }
-            __device__ iterator& operator++() {
-                m.row += F.P.in_record_bytes;
-                if (++m.index >= end_) advance();
-                return *this;
-            }
-            __device__ bool operator!=(const iterator&) const { return m.index < end_; }
-            __device__ bool operator==(const iterator& o) const { return !(*this != o); }
-            __device__ const Message& operator*() const { return m; }
-            __device__ const Message* operator->() const { return &m; }
-
-         private:
-            // hash of cell t of the visit order (x offset outer, z inner)
-            __device__ uint32_t hash(int t) const {
-                if (DIMS == 3)
-                    return pick(t / 9, F.hx0, F.hx1, F.hx2) + pick((t / 3) % 3, F.hy0, F.hy1, F.hy2) +
-                           pick(t % 3, F.hz0, F.hz1, F.hz2);
-                return pick(t / 3, F.hx0, F.hx1, F.hx2) + pick(t % 3, F.hy0, F.hy1, F.hy2);
-            }
-            // bounds of the next non-empty cell (an empty pair when none is left)
-            __device__ void prefetch() {
-                nb_ = ne_ = 0;
-                if (todo_) {
-                    const int t = __ffs(todo_) - 1;
-                    todo_ &= todo_ - 1u;
-                    const uint32_t h = hash(t);
-                    nb_ = F.win.pbm_at(F.P, h);
-                    ne_ = F.win.pbm_at(F.P, h + 1);
-                }
-            }
-            // enter the prefetched cell (index == end ends the loop)
-            __device__ void advance() {
-                m.index = nb_;
-                m.row = F.win.row(F.P, nb_);
-                end_ = ne_;
-                prefetch();  // in flight while this cell is read
-            }
-            const WrapFilter& F;
-            Message m;
-            uint32_t end_;
-            uint32_t todo_ = 0;         // non-empty cells not yet entered
-            uint32_t nb_ = 0, ne_ = 0;  // bounds of the next one
-        };
-        __device__ WrapFilter(const detail::LaunchParams& p, float x, float y, float z) : P(p) {
-            loc[0] = x;
-            loc[1] = y;
-            loc[2] = z;
-            const fg_spatial_grid& gc = detail::ctx().grid;
-            cell[0] = detail::grid_cell(gc, 0, x);
-            cell[1] = detail::grid_cell(gc, 1, y);
-            cell[2] = DIMS == 3 ? detail::grid_cell(gc, 2, z) : 0;
-            // wrapped coordinates of the offsets -1, 0, +1 on each axis (modulo gridDim,
-            // MessageSpatial3DDevice.cuh:736-738), pre-multiplied into hash terms.
-            const fg_spatial_grid& g = detail::ctx().grid;
-            auto wrapc = [](int c, int r, uint32_t d) {
-                return static_cast<uint32_t>(c + r + static_cast<int>(d)) % d;
-            };
-            hx0 = wrapc(cell[0], -1, g.gridDim[0]);
-            hx1 = wrapc(cell[0], 0, g.gridDim[0]);
-            hx2 = wrapc(cell[0], 1, g.gridDim[0]);
-            hy0 = wrapc(cell[1], -1, g.gridDim[1]) * g.gridDim[0];
-            hy1 = wrapc(cell[1], 0, g.gridDim[1]) * g.gridDim[0];
-            hy2 = wrapc(cell[1], 1, g.gridDim[1]) * g.gridDim[0];
-            if (DIMS == 3) {
-                const uint32_t s2 = g.gridDim[0] * g.gridDim[1];
-                hz0 = wrapc(cell[2], -1, g.gridDim[2]) * s2;
-                hz1 = wrapc(cell[2], 0, g.gridDim[2]) * s2;
-                hz2 = wrapc(cell[2], 1, g.gridDim[2]) * s2;
-            } else {
-                hz0 = hz1 = hz2 = 0;
-            }
-            win.load(p);
-        }
-        __device__ iterator begin() const { return iterator(*this, false); }
-        __device__ iterator end() const { return iterator(*this, true); }
-
-        const detail::LaunchParams& P;
-        float loc[3];
-        int cell[3];
-        uint32_t hx0, hx1, hx2, hy0, hy1, hy2, hz0, hz1, hz2;
-        Window win;
-    };
-
-    __device__ explicit SpatialIn(const detail::LaunchParams& p) : P(p) {}
-    __device__ float radius() const { return detail::ctx().grid.radius; }
+    __device__ explicit SpatialIn(const detail::Launch& l) : L(l), P(l.P) {}
+    __device__ float radius() const { return L.grid().radius; }
 
  protected:
     // MessageSpatial3D::In::wrap seatbelts (MessageSpatial3DDevice.cuh:527-549)
     __device__ bool wrap_ok(float x, float y, float z) const {
 #if FLAMEGPU_SEATBELTS
-        const fg_spatial_grid& g = detail::ctx().grid;
+        const fg_spatial_grid& g = L.grid();
         bool out = x > g.max[0] || y > g.max[1] || x < g.min[0] || y < g.min[1];
         if (DIMS == 3) out = out || z > g.max[2] || z < g.min[2];
         if (out) {
@@ -1145,7 +1198,9 @@ class SpatialIn {
 #endif
         return true;
     }
+    const detail::Launch L;
     const detail::LaunchParams& P;
+    mutable bool busy = false;  // a filter of this thread holds its range words
 };
 
 /** MessageSpatial2D (include/flamegpu/runtime/messaging/MessageSpatial2D/MessageSpatial2DDevice.cuh). */
@@ -1154,11 +1209,11 @@ class MessageSpatial2D {
     class Description;
     class In : public SpatialIn<2> {
      public:
-        __device__ explicit In(const detail::LaunchParams& p) : SpatialIn<2>(p) {}
-        __device__ Filter operator()(float x, float y) const { return Filter(P, x, y, 0.0f); }
+        __device__ explicit In(const detail::Launch& l) : SpatialIn<2>(l) {}
+        __device__ Filter operator()(float x, float y) const { return Filter(L, busy, x, y, 0.0f); }
         __device__ WrapFilter wrap(float x, float y) const {
-            if (!wrap_ok(x, y, 0.0f)) return WrapFilter(P, detail::ctx().grid.min[0], detail::ctx().grid.min[1], 0.0f);
-            return WrapFilter(P, x, y, 0.0f);
+            if (!wrap_ok(x, y, 0.0f)) return WrapFilter(L, busy, L.grid().min[0], L.grid().min[1], 0.0f);
+            return WrapFilter(L, busy, x, y, 0.0f);
         }
     };
     class Out : public MessageOutBase {
@@ -1177,11 +1232,11 @@ class MessageSpatial3D {
     class Description;
     class In : public SpatialIn<3> {
      public:
-        __device__ explicit In(const detail::LaunchParams& p) : SpatialIn<3>(p) {}
-        __device__ Filter operator()(float x, float y, float z) const { return Filter(P, x, y, z); }
+        __device__ explicit In(const detail::Launch& l) : SpatialIn<3>(l) {}
+        __device__ Filter operator()(float x, float y, float z) const { return Filter(L, busy, x, y, z); }
         __device__ WrapFilter wrap(float x, float y, float z) const {
-            if (!wrap_ok(x, y, z)) return WrapFilter(P, detail::ctx().grid.min[0], detail::ctx().grid.min[1], detail::ctx().grid.min[2]);
-            return WrapFilter(P, x, y, z);
+            if (!wrap_ok(x, y, z)) return WrapFilter(L, busy, L.grid().min[0], L.grid().min[1], L.grid().min[2]);
+            return WrapFilter(L, busy, x, y, z);
         }
     };
     class Out : public MessageOutBase {
@@ -1370,17 +1425,17 @@ class DeviceMacroProperty {
 /** Read-only environment properties (include/flamegpu/runtime/environment/DeviceEnvironment.cuh). */
 class DeviceEnvironment {
  public:
-    __device__ explicit DeviceEnvironment(const detail::LaunchParams& p) : P(p) {}
+    __device__ explicit DeviceEnvironment(const detail::Launch& l) : L(l), P(l.P) {}
     // env table pointers are offsets into the instance's environment buffer
     template <typename T>
     __device__ T getProperty(detail::VarName name) const {
         const T* off = detail::var_addr<T>(P, &P.T.env, name.hash, 0, 0);
-        return detail::ldg_any(reinterpret_cast<const T*>(detail::ctx().env + reinterpret_cast<size_t>(off)));
+        return detail::ldg_any(reinterpret_cast<const T*>(L.env() + reinterpret_cast<size_t>(off)));
     }
     template <typename T, flamegpu::size_type N>
     __device__ T getProperty(detail::VarName name, unsigned int i) const {
         const T* off = detail::var_addr<T>(P, &P.T.env, name.hash, 0, i);
-        return detail::ldg_any(reinterpret_cast<const T*>(detail::ctx().env + reinterpret_cast<size_t>(off)));
+        return detail::ldg_any(reinterpret_cast<const T*>(L.env() + reinterpret_cast<size_t>(off)));
     }
     /** DeviceEnvironment::getMacroProperty (DeviceEnvironment.cuh:95-112). A
      *  name that is not a macro property of this type and these dimensions is
@@ -1396,12 +1451,13 @@ class DeviceEnvironment {
                                  name.hash, 0);
             return DeviceMacroProperty<T, I, J, K, W>(P, nullptr, nullptr);
         }
-        char* env = const_cast<char*>(detail::ctx().env);
+        char* env = const_cast<char*>(L.env());
         return DeviceMacroProperty<T, I, J, K, W>(P, reinterpret_cast<T*>(env + reinterpret_cast<size_t>(vs->ptr)),
                                                   reinterpret_cast<uint32_t*>(env + vs->stride));
     }
 
  private:
+    const detail::Launch L;
     const detail::LaunchParams& P;
 };
 
@@ -1418,7 +1474,7 @@ class DeviceEnvironment {
  */
 class AgentRandom {
  public:
-    __device__ AgentRandom(const detail::LaunchParams& p, uint32_t idx) : P(p), index(idx) {}
+    __device__ AgentRandom(const detail::Launch& l, uint32_t idx) : L(l), P(l.P), index(idx) {}
     template <typename T>
     __device__ T uniform() const;
     template <typename T>
@@ -1432,9 +1488,10 @@ class AgentRandom {
 
  private:
     __device__ uint64_t next() const {
-        const uint64_t key = detail::mix64(detail::ctx().seed ^ (static_cast<uint64_t>(P.fn_uid) << 40) ^ detail::ctx().step);
+        const uint64_t key = detail::mix64(L.seed() ^ (static_cast<uint64_t>(P.fn_uid) << 40) ^ L.step());
         return detail::mix64(detail::mix64(key + index) + (counter++));
     }
+    const detail::Launch L;
     const detail::LaunchParams& P;
     uint32_t index;
     mutable uint32_t counter = 0;
@@ -1525,7 +1582,7 @@ class DeviceAPI {
     /** agent_out: birth of at most one agent per agent function call (DeviceAPI.cuh:187-236). */
     class AgentOut {
      public:
-        __device__ AgentOut(const detail::LaunchParams& p, uint32_t idx) : P(p), index(idx) {}
+        __device__ AgentOut(const detail::Launch& l, uint32_t idx) : L(l), P(l.P), index(idx) {}
         template <typename T>
         __device__ void setVariable(detail::VarName name, T value) const {
             if (!start(name)) return;
@@ -1544,7 +1601,7 @@ class DeviceAPI {
             if (!start_row(0u)) return ID_NOT_SET;
             if (is_born != 2u) {
                 // a batch keeps one next id per instance
-                claimed = atomicAdd(P.birth_next_id + detail::ctx().inst, 1u);
+                claimed = atomicAdd(P.birth_next_id + L.inst(), 1u);
                 detail::write_var<id_t>(P, &P.T.birth, detail::VarName("_id").hash, index, claimed);
                 is_born = 2u;
             }
@@ -1583,18 +1640,18 @@ class DeviceAPI {
             }
             return true;
         }
+        const detail::Launch L;
         const detail::LaunchParams& P;
         uint32_t index;
         mutable uint32_t is_born = 0;  // 1: born, 2: born and its id claimed
         mutable id_t claimed = ID_NOT_SET;
     };
 
-    __device__ DeviceAPI(const detail::LaunchParams& p, uint32_t idx)
-        : message_in(p), message_out(p, idx), agent_out(p, idx), environment(p), random(p, idx), P(p), index(idx) {}
     /** msg_row: the row this agent's output message takes (the agent's index
      *  among those running the function). */
-    __device__ DeviceAPI(const detail::LaunchParams& p, uint32_t idx, uint32_t msg_row)
-        : message_in(p), message_out(p, msg_row), agent_out(p, idx), environment(p), random(p, idx), P(p), index(idx) {}
+    __device__ DeviceAPI(const detail::Launch& l, uint32_t idx, uint32_t msg_row)
+        : message_in(l), message_out(l, msg_row), agent_out(l, idx), environment(l), random(l, idx), L(l), P(l.P),
+          index(idx) {}
 
     template <typename T>
     __device__ T getVariable(detail::VarName name) const {
@@ -1624,8 +1681,8 @@ class DeviceAPI {
         detail::write_var<T>(P, &P.T.agent, name.hash, index, value, i);
     }
     __device__ id_t getID() const { return detail::read_rw<id_t>(P, &P.T.agent, detail::VarName("_id").hash, index); }
-    __device__ unsigned int getStepCounter() const { return detail::ctx().step; }
-    __device__ unsigned int getIndex() const { return index - detail::ctx().row_begin; }
+    __device__ unsigned int getStepCounter() const { return L.step(); }
+    __device__ unsigned int getIndex() const { return index - L.row_begin(); }
     /** Whether the function runs on agents of this name / in this state
      *  (DeviceAPI.cuh:366-380 of the reference; names compared by hash). */
     __device__ bool isAgent(const char* agent_name) const { return detail::fnv1a32(agent_name, ~0u) == P.agent_hash; }
@@ -1642,6 +1699,7 @@ class DeviceAPI {
     uint32_t pos_set = 0;
 
  private:
+    const detail::Launch L;
     const detail::LaunchParams& P;
     uint32_t index;
 };
@@ -1651,8 +1709,8 @@ class DeviceAPI {
  *  counter, environment properties and random numbers; nothing is written. */
 class ReadOnlyDeviceAPI {
  public:
-    __device__ ReadOnlyDeviceAPI(const detail::LaunchParams& p, uint32_t idx)
-        : environment(p), random(p, idx), P(p), index(idx) {}
+    __device__ ReadOnlyDeviceAPI(const detail::Launch& l, uint32_t idx)
+        : environment(l), random(l, idx), L(l), P(l.P), index(idx) {}
     template <typename T>
     __device__ T getVariable(detail::VarName name) const {
         return detail::read_rw<T>(P, &P.T.agent, name.hash, index);
@@ -1662,8 +1720,8 @@ class ReadOnlyDeviceAPI {
         return detail::read_rw<T>(P, &P.T.agent, name.hash, index, i);
     }
     __device__ id_t getID() const { return detail::read_rw<id_t>(P, &P.T.agent, detail::VarName("_id").hash, index); }
-    __device__ unsigned int getStepCounter() const { return detail::ctx().step; }
-    __device__ unsigned int getIndex() const { return index - detail::ctx().row_begin; }
+    __device__ unsigned int getStepCounter() const { return L.step(); }
+    __device__ unsigned int getIndex() const { return index - L.row_begin(); }
     __device__ bool isAgent(const char* agent_name) const { return detail::fnv1a32(agent_name, ~0u) == P.agent_hash; }
     __device__ bool isState(const char* agent_state) const { return detail::fnv1a32(agent_state, ~0u) == P.state_hash; }
 
@@ -1671,6 +1729,7 @@ class ReadOnlyDeviceAPI {
     AgentRandom random;
 
  private:
+    const detail::Launch L;
     const detail::LaunchParams& P;
     uint32_t index;
 };
