@@ -1,4 +1,4 @@
-// Device helpers shared by the GB300 kernels: acquire/release accesses for the
+// Device helpers shared by the GB300 kernels: the tile-status accesses of the
 // single-pass scans, bounded waits, the workspace header and launch sizing.
 #pragma once
 
@@ -59,18 +59,18 @@ static_assert(offsetof(WsHeader, long_count) == 4 * flamegpu::detail::kWsHdrLong
 static_assert(offsetof(WsHeader, key_max) == 4 * flamegpu::detail::kWsHdrKeyMax, "header layout");
 static_assert(offsetof(WsHeader, disorder) == 4 * flamegpu::detail::kWsHdrDisorder, "header layout");
 
-__device__ __forceinline__ uint64_t ld_acquire_u64(const uint64_t* p) {
+// Tile statuses of the look-backs. A status is one 64-bit word that holds all
+// its reader needs, so it is published and read relaxed: no other memory is
+// handed over with it. (A release store waits for a fence, and an acquire
+// load drops L1: an agent sort of 16,384 rows took 17.3 us with them, 16.6
+// without.)
+__device__ __forceinline__ uint64_t ld_status(const uint64_t* p) {
     uint64_t v;
-    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
     return v;
 }
-__device__ __forceinline__ void st_release_u64(uint64_t* p, uint64_t v) {
-    asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-__device__ __forceinline__ uint32_t ld_acquire_u32(const uint32_t* p) {
-    uint32_t v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
+__device__ __forceinline__ void st_status(uint64_t* p, uint64_t v) {
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 // Read-only load (data not written while the kernel runs); not volatile, so
 // the compiler may schedule several before their first use.

@@ -68,7 +68,7 @@ __device__ __forceinline__ uint32_t lookback_u32(const uint64_t* status, uint32_
         if (t >= 0) {
             uint32_t spins = 0, limit = 0xFFFFFFFFu;
             for (;;) {
-                const uint64_t s = ld_acquire_u64(status + t);
+                const uint64_t s = ld_status(status + t);
                 const uint32_t e = static_cast<uint32_t>(s >> 32) & 0x3FFFFFFFu;
                 flag = static_cast<uint32_t>(s >> 62);
                 val = static_cast<uint32_t>(s);
@@ -211,11 +211,11 @@ __device__ __forceinline__ bool scan_tile(const ScanJob& j, uint32_t tile, uint3
     if (threadIdx.x < 32) {
         uint32_t excl = 0;
         if (tile == 0) {
-            if (threadIdx.x == 0 && !withhold) st_release_u64(j.status, scan_pack(2, epoch, ttotal));
+            if (threadIdx.x == 0 && !withhold) st_status(j.status, scan_pack(2, epoch, ttotal));
         } else {
-            if (threadIdx.x == 0) st_release_u64(j.status + tile, scan_pack(1, epoch, ttotal));
+            if (threadIdx.x == 0) st_status(j.status + tile, scan_pack(1, epoch, ttotal));
             excl = lookback_u32(j.status, tile, epoch, j.h);
-            if (threadIdx.x == 0) st_release_u64(j.status + tile, scan_pack(2, epoch, excl + ttotal));
+            if (threadIdx.x == 0) st_status(j.status + tile, scan_pack(2, epoch, excl + ttotal));
         }
         if (threadIdx.x == 0) *s_excl = excl;
     }
@@ -260,8 +260,8 @@ __device__ __forceinline__ bool scan_tile(const ScanJob& j, uint32_t tile, uint3
 }
 
 // Thread 0: the block's tile (ticket), the scan's epoch, and the test hook
-// and order-check state. The key launch's flag is final (it completed before
-// this launch): read before the acquire, so the loads overlap.
+// and order-check state. All of it is final (earlier launches wrote it), so
+// the loads overlap the ticket's atomic.
 struct ScanTicket {
     uint32_t tile, epoch, withhold, pending;
 };
@@ -269,7 +269,7 @@ __device__ __forceinline__ ScanTicket scan_ticket_of(const ScanJob& j, uint32_t 
     ScanTicket t;
     t.pending = j.oc.edges != nullptr && j.h->disorder == 0u;
     t.tile = ticket;
-    t.epoch = ld_acquire_u32(&j.h->scan_epoch);
+    t.epoch = j.h->scan_epoch;
     t.withhold = ticket == 0 ? j.h->withhold : 0u;
     return t;
 }
