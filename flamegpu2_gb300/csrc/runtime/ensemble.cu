@@ -593,17 +593,19 @@ struct BatchedSim {
             }
             if (b.births) {
                 e.clear();
-                std::vector<TableEntry> d;
-                size_t doff = 0;
+                std::vector<size_t> doff;
+                size_t at = 0;
                 for (size_t v = 0; v < agent->variables.size(); ++v) {
                     const Variable& var = agent->variables[v];
                     e.push_back({fnv1a32(var.name), static_cast<char*>(b.birth_cols[v]), var.bytes(), var.type_size, var.elements});
-                    d.push_back({fnv1a32(var.name), static_cast<char*>(b.birth_defaults) + doff, var.bytes(), var.type_size,
-                                 var.elements});
-                    doff = (doff + var.default_value.size() + 7) & ~size_t(7);
+                    doff.push_back(at);
+                    at = (at + var.default_value.size() + 7) & ~size_t(7);
                 }
                 T->birth = make_table(e, "agent");
-                T->birth_def = make_table(d, "agent");
+                for (size_t v = 0; v < agent->variables.size(); ++v)
+                    T->birth_default[T->birth_defaults++] =
+                        birth_default(b.birth_cols[v], agent->variables[v].bytes(),
+                                      static_cast<char*>(b.birth_defaults) + doff[v], agent->variables[v].default_value.data());
             }
             e.clear();
             for (size_t i = 0; i < model->environment.size(); ++i) {

@@ -3,6 +3,7 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <cstring>
 #include <vector>
 
 #include "flamegpu/detail/device_types.cuh"
@@ -21,6 +22,19 @@ struct TableEntry {
 /** Collision-free multiplicative lookup table over the given variables:
  * slot = (hash * mult) >> shift; throws if no multiplier up to 64 slots works. */
 VarTable make_table(const std::vector<TableEntry>& e, const char* what);
+
+/** The default of a birth variable: column, its staging rows (8-byte aligned);
+ * device_value, the default's bytes on the device; value, the same on the host. */
+inline BirthDefault birth_default(void* column, uint32_t bytes, const void* device_value, const void* value) {
+    BirthDefault d{};
+    d.column = static_cast<char*>(column);
+    d.bytes = bytes;
+    if (bytes == 4u || bytes == 8u)
+        std::memcpy(&d.value, value, bytes);
+    else
+        d.value = reinterpret_cast<uint64_t>(device_value);
+    return d;
+}
 
 /** Layout of a spatial message record: the location (x, y[, z], 4 bytes
  *  each) at words 0..dims-1, then every other variable at word

@@ -1121,7 +1121,6 @@ struct SimulationImpl {
             }
             if (f.births) {
                 e.clear();
-                std::vector<TableEntry> d;
                 std::vector<char> defaults;
                 std::vector<size_t> doff;
                 const AgentData* ba = f.birth_list->agent;
@@ -1135,10 +1134,12 @@ struct SimulationImpl {
                 for (size_t v = 0; v < ba->variables.size(); ++v) {
                     const Variable& var = ba->variables[v];
                     e.push_back({fnv1a32(var.name), static_cast<char*>(f.birth_cols[v]), var.bytes(), var.type_size, var.elements});
-                    d.push_back({fnv1a32(var.name), static_cast<char*>(f.birth_defaults) + doff[v], var.bytes(), var.type_size, var.elements});
                 }
                 T->birth = make_table(e, "agent");
-                T->birth_def = make_table(d, "agent");
+                for (size_t v = 0; v < ba->variables.size(); ++v)
+                    T->birth_default[T->birth_defaults++] =
+                        birth_default(f.birth_cols[v], ba->variables[v].bytes(),
+                                      static_cast<char*>(f.birth_defaults) + doff[v], ba->variables[v].default_value.data());
             }
             e.clear();
             for (size_t i = 0; i < model->environment.size(); ++i) {

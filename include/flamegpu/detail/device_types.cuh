@@ -62,13 +62,23 @@ __host__ __device__ inline uint32_t table_slot(uint32_t mult, uint32_t shift, ui
     return (hash * mult) >> shift;
 }
 
+/** The default of one variable of agent_out's agent: what a birth's staging row holds until the function sets it. */
+struct BirthDefault {
+    char* column;     // staging rows, `bytes` apart
+    uint32_t bytes;
+    uint32_t pad;
+    uint64_t value;   // 4- and 8-byte variables: the value itself; others: its address (device)
+};
+
 /** Read-only tables of one agent function launch (kernel parameters). */
 struct FunctionTables {
     VarTable agent;      // the agent's own variables (SoA columns)
     VarTable msg_out;    // output message list (unsorted SoA columns)
     VarTable msg_in;     // input message list (sorted records, or SoA for brute force)
     VarTable birth;      // agent_out staging rows (SoA, indexed by parent)
-    VarTable birth_def;  // default value of each agent_out variable (ptr -> value bytes)
+    uint32_t birth_defaults;  // agent_out's variables, in declaration order
+    uint32_t pad;
+    BirthDefault birth_default[kMaxVarSlots];
     VarTable env;        // environment properties (ptr -> value bytes)
 };
 
