@@ -27,7 +27,7 @@ constexpr int kThreads = 256;
 
 // Default upper bound on polls of one predecessor's status in a decoupled
 // look-back. A predecessor tile always belongs to a block that is already
-// running (tiles are handed out in launch order by a ticket counter), so the
+// running (tiles go to blocks in launch order), so the
 // wait ends in practice within microseconds; the bound only turns a broken
 // invariant into a recorded error instead of a hung GPU (~2^22 polls with
 // backoff ≈ 1-2 s). A workspace header may carry a smaller bound
@@ -38,7 +38,7 @@ constexpr uint32_t kSpinLimit = 1u << 22;
 struct WsHeader {
     uint32_t status;        // fg_status recorded on the device (0 = OK)
     uint32_t scan_epoch;    // generation tag of the scan tile statuses
-    uint32_t scan_ticket;   // tile ticket counter of the scan
+    uint32_t unused;
     uint32_t scan_done;     // finished scan blocks (last one resets)
     uint32_t long_count;    // long bins queued for the segment stabiliser
     uint32_t comp_ticket;   // compaction tile tickets
@@ -54,7 +54,6 @@ struct WsHeader {
 static_assert(sizeof(WsHeader) == 256, "header is 256 bytes");
 // words an agent-function launch resets when it computes a build's keys
 static_assert(offsetof(WsHeader, scan_epoch) == 4 * flamegpu::detail::kWsHdrScanEpoch, "header layout");
-static_assert(offsetof(WsHeader, scan_ticket) == 4 * flamegpu::detail::kWsHdrScanTicket, "header layout");
 static_assert(offsetof(WsHeader, long_count) == 4 * flamegpu::detail::kWsHdrLongCount, "header layout");
 static_assert(offsetof(WsHeader, key_max) == 4 * flamegpu::detail::kWsHdrKeyMax, "header layout");
 static_assert(offsetof(WsHeader, disorder) == 4 * flamegpu::detail::kWsHdrDisorder, "header layout");

@@ -193,19 +193,27 @@ struct PermJob {
     WsHeader* h;
 };
 
-// By block b of the nb blocks working on job j.
+// By block b of the nb blocks working on job j. A row's key and slot are read
+// one round ahead (the first beside the count and the order flag).
 __device__ __forceinline__ void perm_rows(const PermJob& j, uint32_t b, uint32_t nb) {
-    if (j.h->disorder == 0u) return;  // keys in row order: every row keeps its place
+    const uint32_t stride = nb * blockDim.x;
+    uint32_t i = b * blockDim.x + threadIdx.x;
+    uint32_t k = i < j.max_n ? j.keys[i] : kInvalid, slot = i < j.max_n ? j.slot[i] : 0u;
     const uint32_t n = load_count(j.d_n, j.max_n);
-    for (uint32_t i = b * blockDim.x + threadIdx.x; i < n; i += nb * blockDim.x) {
-        const uint32_t k = j.keys[i];
+    if (j.h->disorder == 0u) return;  // keys in row order: every row keeps its place
+    while (i < n) {
+        const uint32_t next = i + stride;
+        const uint32_t nk = next < n ? j.keys[next] : kInvalid, ns = next < n ? j.slot[next] : 0u;
         if (k != kInvalid) {
-            const uint32_t at = j.pbm[k & ~kPadBit] + j.slot[i];
+            const uint32_t at = j.pbm[k & ~kPadBit] + slot;
             if (at < n)
                 j.perm[at] = i;
             else
                 record_status(j.h, FG_ERR_WORKSPACE);
         }
+        i = next;
+        k = nk;
+        slot = ns;
     }
 }
 
@@ -396,10 +404,10 @@ __device__ __forceinline__ void emit_run(const EmitParams& ep, uint32_t* sperm, 
 // What the stabilising and long-bin kernels of one counting sort read and
 // write: the emission, the keys, PBM and unstable placement, the stable
 // permutation (agent sorts), the long-bin chunk queue, the workspace header,
-// and for agent sorts the recorded largest key (key_max) and its floor.
+// the number of sorted rows (device, at most max_n; null: max_n), and for
+// agent sorts the recorded largest key, which k_long clears.
 struct StabJob {
     EmitParams rp;
-    uint32_t nbuckets;
     const uint32_t* keys;
     const uint32_t* pbm;
     const uint32_t* perm;
@@ -408,27 +416,30 @@ struct StabJob {
     uint32_t chunk_cap;
     WsHeader* h;
     uint32_t* key_max;
-    uint32_t key_floor;
+    const uint32_t* total;
     uint32_t max_n;
 };
 
-// Sorted positions p < total = pbm[nbuckets] (for an agent sort, whose scan
-// stopped past max(recorded key, cells - 1), the PBM entry after that). Short bins are ranked in place
-// (count of smaller original indices in the bin); long bins are queued as
-// chunks (bucket, chunk index) for k_long.
+// Sorted positions p < total (*total of the job). Short bins are ranked in
+// place (count of smaller original indices in the bin); long bins are queued
+// as chunks (bucket, chunk index) for k_long. A position's entry is read one
+// round ahead (the first beside the total and the order flag).
 template <int EMIT>
 __device__ __forceinline__ void stabilize_positions(const StabJob& j, uint32_t blk, uint32_t nblk) {
-    // key_max (agent sorts): the PBM ends at max(recorded key, key_floor) + 1
-    const uint32_t total = j.pbm[j.key_max ? min(j.nbuckets, max(*j.key_max, j.key_floor) + 1u) : j.nbuckets];
+    const uint32_t stride = nblk * blockDim.x;
+    uint32_t p = blk * blockDim.x + threadIdx.x;
+    uint32_t ahead = p < j.max_n ? j.perm[p] : 0u;
+    const uint32_t total = load_count(j.total, j.max_n);
     if (j.h->disorder == 0u) {
         // keys in row order (the key launch and the scan found no descent):
         // the stable order is the row order, so rows are emitted in place, as
         // one run over the grid's threads (four rows in flight per thread)
-        emit_run<EMIT>(j.rp, j.sperm, 0u, 0u, min(total, j.max_n), blk * blockDim.x + threadIdx.x, nblk * blockDim.x);
+        emit_run<EMIT>(j.rp, j.sperm, 0u, 0u, total, p, stride);
         return;
     }
-    for (uint32_t p = blk * blockDim.x + threadIdx.x; p < total; p += nblk * blockDim.x) {
-        const uint32_t i = j.perm[p];
+    for (; p < total; p += stride) {
+        const uint32_t i = ahead;
+        ahead = p + stride < total ? j.perm[p + stride] : 0u;
         const uint32_t b = j.keys[i];
         if (b & kPadBit) {  // padding row of a batch: keeps its slot, carries no message
             if (EMIT != kEmitRecord) j.sperm[p] = i;
@@ -932,7 +943,10 @@ int run_pipeline(const fg_spatial_grid* g, const SortGrid& sg, uint32_t nbuckets
     const OrderCheck oc{batch.inst ? nullptr : edges, d_n, max_n};
     launch_scan(hist, pbm_out, scan_n, 1, sstat, h, 0, st, key_max, key_floor, oc);
     launch(k_perm, grid, kThreads, st, PermJob{max_n, d_n, keys, slot, pbm_out, perm, h});
-    const StabJob sj{rp, nbuckets, keys, pbm_out, perm, sperm, chunks, L.chunk_cap, h, key_max, key_floor, max_n};
+    // every row of an agent sort and of a batch (padding rows too) has a bucket;
+    // a list's messages are counted by its PBM
+    const uint32_t* total = MODE == kSortKey || batch.inst ? d_n : pbm_out + nbuckets;
+    const StabJob sj{rp, keys, pbm_out, perm, sperm, chunks, L.chunk_cap, h, key_max, total, max_n};
     launch(k_stabilize<EMIT>, grid, kThreads, st, sj);
     launch(k_long<EMIT>, long_grid_for(max_n), kThreads, st, sj);
     return check_launch();
@@ -1046,10 +1060,10 @@ int fgi_spatial_sort_and_build(const fg_spatial_grid* g, uint32_t sort_max_n, co
     launch(k_perm_pair, ga + gb, kThreads, st, PermJob{sort_max_n, sort_d_n, at(wa, La.keys), at(wa, La.slot), pbm_a,
                                                        at(wa, La.perm), ha},
            PermJob{msg_max_n, msg_d_n, at(wb, Lb.keys), at(wb, Lb.slot), pbm, at(wb, Lb.perm), hb}, ga);
-    const StabJob ja{ea, nb, at(wa, La.keys), pbm_a, at(wa, La.perm), at(wa, La.sperm),
-                     reinterpret_cast<uint2*>(wa + La.chunks), La.chunk_cap, ha, &ha->key_max, key_floor, sort_max_n};
-    const StabJob jb{eb, g->binCount, at(wb, Lb.keys), pbm, at(wb, Lb.perm), nullptr,
-                     reinterpret_cast<uint2*>(wb + Lb.chunks), Lb.chunk_cap, hb, nullptr, 0, msg_max_n};
+    const StabJob ja{ea, at(wa, La.keys), pbm_a, at(wa, La.perm), at(wa, La.sperm),
+                     reinterpret_cast<uint2*>(wa + La.chunks), La.chunk_cap, ha, &ha->key_max, sort_d_n, sort_max_n};
+    const StabJob jb{eb, at(wb, Lb.keys), pbm, at(wb, Lb.perm), nullptr,
+                     reinterpret_cast<uint2*>(wb + Lb.chunks), Lb.chunk_cap, hb, nullptr, pbm + g->binCount, msg_max_n};
     launch(k_stabilize_pair<kEmitPermColumns, kEmitRecord>, ga + gb, kThreads, st, ja, jb, ga);
     const uint32_t la = long_grid_for(sort_max_n), lb = long_grid_for(msg_max_n);
     launch(k_long_pair<kEmitPermColumns, kEmitRecord>, la + lb, kThreads, st, ja, jb, la);
