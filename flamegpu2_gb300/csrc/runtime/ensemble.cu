@@ -738,7 +738,9 @@ struct BatchedSim {
             const fg_spatial_grid& g = m.inst[k].grid;
             const double per_bin = static_cast<double>(count[k]) / std::max<uint32_t>(g.binCount, 1u);
             all += count[k];
-            if (detail::stage_window_fits(g, per_bin, m.record_words, shape.block, shape.stage_bytes)) fit += count[k];
+            if (detail::stage_window_fits(g, per_bin, m.record_words, shape.block, shape.stage_bytes, total_rows / shape.block,
+                                          static_cast<uint32_t>(sms)))
+                fit += count[k];
         }
         return all > 0.0 && fit >= 0.5 * all;
     }

@@ -1641,9 +1641,13 @@ struct SimulationImpl {
     // per block, never a wrong result; a population far below its capacity
     // (a decaying birth/death run) launches few blocks. The step graphs are
     // keyed by it, so a change of class captures a graph sized for it.
-    uint32_t grid_rows(const AgentList& l) const {
+    static uint32_t population_class(const AgentList& l) {
         uint64_t r = 1;
         while (r < l.bound) r <<= 1;
+        return static_cast<uint32_t>(std::min<uint64_t>(r, 0xFFFFFFFFull));
+    }
+    uint32_t grid_rows(const AgentList& l) const {
+        uint64_t r = population_class(l);
         r = std::max<uint64_t>(r, 8ull * static_cast<uint64_t>(sms) * kAgentBlock);
         return static_cast<uint32_t>(std::min<uint64_t>(r, std::max(l.capacity, 1u)));
     }
@@ -1666,9 +1670,9 @@ struct SimulationImpl {
         return std::min(std::max(1u, (rows + block - 1) / block), 1u << 17);
     }
 
-    static bool stage_window_fits(const MsgList& m, unsigned int stage_bytes, unsigned int block) {
+    bool stage_window_fits(const MsgList& m, unsigned int stage_bytes, unsigned int block, unsigned int blocks) const {
         const double per_bin = static_cast<double>(m.capacity) / std::max<uint32_t>(m.grid.binCount, 1u);
-        return detail::stage_window_fits(m.grid, per_bin, m.record_words, block, stage_bytes);
+        return detail::stage_window_fits(m.grid, per_bin, m.record_words, block, stage_bytes, blocks, sms);
     }
 
     void enqueue_function(FnRt& f) {
@@ -1775,7 +1779,8 @@ struct SimulationImpl {
                 P.in_index_bits = detail::index_bits(f.in->capacity);
                 P.in_pbm_alloc = f.in->pbm_alloc;
                 if (f.stage && cuda_config.message_stage_bytes >= 1024u &&
-                    stage_window_fits(*f.in, cuda_config.message_stage_bytes, agent_block(grid_rows(l))))
+                    stage_window_fits(*f.in, cuda_config.message_stage_bytes, agent_block(grid_rows(l)),
+                                      agent_grid(std::min(population_class(l), l.capacity), agent_block(grid_rows(l)))))
                     P.stage_bytes = (cuda_config.message_stage_bytes + 15u) & ~15u;
             } else if (f.in->array()) {
                 P.in_count = f.in->arr_count;

@@ -68,3 +68,23 @@ def test_nested_and_copied_searches(dims, n, wrap):
     np.testing.assert_array_equal(s.get("agent", "copied", np.uint32), around[got])
     np.testing.assert_array_equal(s.get("agent", "inner", np.uint32), _neighbourhood_sums(counts * around, wrap)[got])
     s.close()
+
+
+@pytest.mark.parametrize("wrap", [False, True])
+@pytest.mark.parametrize("n", [1, 129, 304 * 128, 304 * 128 + 1])
+def test_staged_and_unstaged_walks_agree(n, wrap):
+    # two blocks of 128 agents a SM are the most that a launch stages windows for
+    from flamegpu2_gb300 import sim, synth
+    cells = max(4, int(np.ceil(n ** (1.0 / 3.0))))
+    cfg = dict(synth.BOIDS_SMALL, n=n, max_pos=2.0 * cells, wrap=int(wrap))
+    pop = synth.boids_population(n, 0.0, 2.0 * cells, 9)
+    got = []
+    for stage in (96 * 1024, 0):
+        s = sim.Simulation("boids_spatial3d", synth.boids_params(cfg))
+        s.set_stage_bytes(stage)
+        s.set_population("Boid", n, pop)
+        s.step(3)
+        got.append([s.get("Boid", "_id", np.uint32)] + [s.get("Boid", k, np.float32) for k in ("x", "y", "z", "fx", "fy", "fz")])
+        s.close()
+    for a, b in zip(*got):
+        np.testing.assert_array_equal(a, b)
