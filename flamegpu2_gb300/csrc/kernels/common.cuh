@@ -38,7 +38,7 @@ constexpr uint32_t kSpinLimit = 1u << 22;
 struct WsHeader {
     uint32_t status;        // fg_status recorded on the device (0 = OK)
     uint32_t scan_epoch;    // generation tag of the scan tile statuses
-    uint32_t unused;
+    uint32_t far_rows;      // rows an agent sort places far from the row before them
     uint32_t scan_done;     // finished scan blocks (last one resets)
     uint32_t long_count;    // long bins queued for the segment stabiliser
     uint32_t comp_ticket;   // compaction tile tickets
@@ -54,6 +54,7 @@ struct WsHeader {
 static_assert(sizeof(WsHeader) == 256, "header is 256 bytes");
 // words an agent-function launch resets when it computes a build's keys
 static_assert(offsetof(WsHeader, scan_epoch) == 4 * flamegpu::detail::kWsHdrScanEpoch, "header layout");
+static_assert(offsetof(WsHeader, far_rows) == 4 * flamegpu::detail::kWsHdrFarRows, "header layout");
 static_assert(offsetof(WsHeader, long_count) == 4 * flamegpu::detail::kWsHdrLongCount, "header layout");
 static_assert(offsetof(WsHeader, key_max) == 4 * flamegpu::detail::kWsHdrKeyMax, "header layout");
 static_assert(offsetof(WsHeader, disorder) == 4 * flamegpu::detail::kWsHdrDisorder, "header layout");

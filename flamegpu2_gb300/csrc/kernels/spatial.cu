@@ -71,6 +71,7 @@ __global__ void __launch_bounds__(kThreads) k_bin(fg_spatial_grid g, SortGrid sg
     flamegpu::detail::grid_dependency_enter();
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         h->long_count = 0;
+        h->far_rows = 0;
         scan_reset(h);  // for the scan launched next
     }
     const uint32_t n = load_count(d_n, max_n);
@@ -204,6 +205,20 @@ __global__ void __launch_bounds__(kThreads) k_bin_batched(const fg_batch_instanc
     }
 }
 
+// An agent sort of more column bytes than L2 holds, of rows in no order: the
+// stabilising kernels then write the stable permutation alone, and
+// k_gather_columns moves the columns by it, one after another, so that the
+// column being gathered (67 MB at 16,777,216 rows) stays in L2. All columns of
+// a row at once fetch DRAM for every 4 bytes: 2,274 us for 16,777,216 rows of
+// seven 4-byte columns, against 185 for the permutation and 950 for the columns.
+// Which way a sort goes is counted by its placement: rows that land more than
+// kFarRows from the row before them are half of all or more when there is no
+// order, few when agents have moved since the last sort (the columns' reads
+// are then nearly in order, and reading the permutation again for every
+// column would cost more than all of them).
+constexpr uint32_t kFarRows = 4096;
+__device__ __forceinline__ bool rows_in_no_order(const WsHeader* h, uint32_t n) { return h->far_rows > n / 2u; }
+
 // One counting sort's placement: perm[PBM[key] + slot] = row.
 struct PermJob {
     uint32_t max_n;
@@ -213,6 +228,7 @@ struct PermJob {
     const uint32_t* pbm;
     uint32_t* perm;
     WsHeader* h;
+    uint32_t count_far;  // count the rows placed far from the row before them (h->far_rows)
 };
 
 // By block b of the nb blocks working on job j. A row's key and slot are read
@@ -223,19 +239,29 @@ __device__ __forceinline__ void perm_rows(const PermJob& j, uint32_t b, uint32_t
     uint32_t k = i < j.max_n ? j.keys[i] : kInvalid, slot = i < j.max_n ? j.slot[i] : 0u;
     const uint32_t n = load_count(j.d_n, j.max_n);
     if (j.h->disorder == 0u) return;  // keys in row order: every row keeps its place
+    uint32_t far = 0;
     while (i < n) {
         const uint32_t next = i + stride;
         const uint32_t nk = next < n ? j.keys[next] : kInvalid, ns = next < n ? j.slot[next] : 0u;
+        uint32_t at = 0;
         if (k != kInvalid) {
-            const uint32_t at = j.pbm[k & ~kPadBit] + slot;
+            at = j.pbm[k & ~kPadBit] + slot;
             if (at < n)
                 j.perm[at] = i;
             else
                 record_status(j.h, FG_ERR_WORKSPACE);
         }
+        if (j.count_far) {
+            const uint32_t before = __shfl_up_sync(__activemask(), at, 1);
+            far += (lane_id() > 0u && (at > before ? at - before : before - at) > kFarRows) ? 1u : 0u;
+        }
         i = next;
         k = nk;
         slot = ns;
+    }
+    if (j.count_far) {
+        far = __reduce_add_sync(__activemask(), far);
+        if (far && lane_id() == static_cast<uint32_t>(__ffs(__activemask()) - 1)) atomicAdd(&j.h->far_rows, far);
     }
 }
 
@@ -289,10 +315,24 @@ __device__ __forceinline__ void record_words8(const RecordParams& rp, uint32_t i
 }
 
 struct ColumnParams {
-    fg_column col[FG_MAX_COLUMNS];
+    fg_column col[FG_MAX_COLUMNS];  // the 4-byte columns, then the 8-byte ones, then the others
     uint32_t ncols;
-    uint32_t keep_perm;  // also write the stable permutation (the caller asked for it)
+    uint32_t nwords, ndoubles;      // how many of the first two
+    uint32_t keep_perm;             // also write the stable permutation (the caller asked for it)
 };
+
+// Columns in the order ColumnParams keeps them (a sort moves every column the
+// same way, so their order is free).
+inline void set_columns(ColumnParams& cp, const fg_column* cols, uint32_t ncols) {
+    cp.ncols = cp.nwords = cp.ndoubles = 0;
+    for (uint32_t c = 0; c < ncols; ++c)
+        if (cols[c].elem_bytes == 4u) cp.col[cp.nwords++] = cols[c];
+    for (uint32_t c = 0; c < ncols; ++c)
+        if (cols[c].elem_bytes == 8u) cp.col[cp.nwords + cp.ndoubles++] = cols[c];
+    cp.ncols = cp.nwords + cp.ndoubles;
+    for (uint32_t c = 0; c < ncols; ++c)
+        if (cols[c].elem_bytes != 4u && cols[c].elem_bytes != 8u) cp.col[cp.ncols++] = cols[c];
+}
 
 template <typename T>
 __device__ __forceinline__ void copy_elem(const void* in, void* out, uint32_t src, uint32_t dst) {
@@ -326,35 +366,65 @@ struct EmitParams {
     ColumnParams cp;
 };
 
-// Every agent column's element i written at dst. Runs of four 4-byte columns
-// (the common float / int variables) are all loaded before any is stored, so
-// their latencies overlap; other columns are copied one by one.
+// Every agent column's element i written at dst. The first eight 4-byte and
+// two 8-byte columns are all loaded before any is stored, so their latencies
+// overlap (2,000,003 agents of seven 4-byte, one 8-byte and one 1-byte column,
+// drifted from their last sort: four columns at a time, mixed widths one by
+// one, took 72 us in k_stabilize, 43 us now).
 __device__ __forceinline__ void emit_columns(const ColumnParams& cp, uint32_t i, uint32_t dst) {
-    for (uint32_t c0 = 0; c0 < cp.ncols; c0 += 4) {
-        const uint32_t nk = min(4u, cp.ncols - c0);
-        bool words = true;
-        for (uint32_t k = 0; k < nk; ++k) words = words && cp.col[c0 + k].elem_bytes == 4u;
-        if (words) {
-            uint32_t v[4];
+    const fg_column* dbl = cp.col + cp.nwords;
+    uint32_t v[8];
+    uint2 w[2];
 #pragma unroll
-            for (uint32_t k = 0; k < 4; ++k)
-                if (k < nk) v[k] = static_cast<const uint32_t*>(cp.col[c0 + k].in)[i];
+    for (uint32_t k = 0; k < 8; ++k)
+        if (k < cp.nwords) v[k] = static_cast<const uint32_t*>(cp.col[k].in)[i];
 #pragma unroll
-            for (uint32_t k = 0; k < 4; ++k)
-                if (k < nk) static_cast<uint32_t*>(cp.col[c0 + k].out)[dst] = v[k];
-        } else {
-            for (uint32_t k = 0; k < nk; ++k) copy_column_elem(cp.col[c0 + k], i, dst);
-        }
+    for (uint32_t k = 0; k < 2; ++k)
+        if (k < cp.ndoubles) w[k] = static_cast<const uint2*>(dbl[k].in)[i];
+#pragma unroll
+    for (uint32_t k = 0; k < 8; ++k)
+        if (k < cp.nwords) static_cast<uint32_t*>(cp.col[k].out)[dst] = v[k];
+#pragma unroll
+    for (uint32_t k = 0; k < 2; ++k)
+        if (k < cp.ndoubles) static_cast<uint2*>(dbl[k].out)[dst] = w[k];
+    for (uint32_t c0 = 8; c0 < cp.nwords; c0 += 4) {
+        const uint32_t nk = min(4u, cp.nwords - c0);
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k)
+            if (k < nk) v[k] = static_cast<const uint32_t*>(cp.col[c0 + k].in)[i];
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k)
+            if (k < nk) static_cast<uint32_t*>(cp.col[c0 + k].out)[dst] = v[k];
     }
+    for (uint32_t c = cp.nwords + min(2u, cp.ndoubles); c < cp.ncols; ++c) copy_column_elem(cp.col[c], i, dst);
 }
 
+// split: only the index, the columns follow by it (k_gather_columns).
 template <int EMIT>
-__device__ __forceinline__ void emit(const EmitParams& ep, uint32_t* sperm, uint32_t i, uint32_t dst) {
+__device__ __forceinline__ void emit(const EmitParams& ep, uint32_t* sperm, uint32_t i, uint32_t dst,
+                                     bool split = false) {
     if (EMIT == kEmitRecord) {
         emit_record(ep.rp, i, dst);
     } else {
-        if (EMIT == kEmitPerm || ep.cp.keep_perm) sperm[dst] = i;
-        if (EMIT == kEmitPermColumns) emit_columns(ep.cp, i, dst);
+        if (EMIT == kEmitPerm || ep.cp.keep_perm || split) sperm[dst] = i;
+        if (EMIT == kEmitPermColumns && !split) emit_columns(ep.cp, i, dst);
+    }
+}
+
+// Elements lo .. lo + len - 1 of a column to s .. s + len - 1, four in flight per thread.
+template <typename T>
+__device__ __forceinline__ void copy_run(const fg_column& c, uint32_t lo, uint32_t s, uint32_t len, uint32_t t,
+                                         uint32_t nt) {
+    const T* in = static_cast<const T*>(c.in) + lo;
+    T* out = static_cast<T*>(c.out) + s;
+    for (uint32_t k0 = t; k0 < len; k0 += 4 * nt) {
+        T v[4];
+#pragma unroll
+        for (uint32_t m = 0; m < 4; ++m)
+            if (k0 + m * nt < len) v[m] = in[k0 + m * nt];
+#pragma unroll
+        for (uint32_t m = 0; m < 4; ++m)
+            if (k0 + m * nt < len) out[k0 + m * nt] = v[m];
     }
 }
 
@@ -365,7 +435,7 @@ __device__ __forceinline__ void emit(const EmitParams& ep, uint32_t* sperm, uint
 // loads in flight instead of one.
 template <int EMIT>
 __device__ __forceinline__ void emit_run(const EmitParams& ep, uint32_t* sperm, uint32_t lo, uint32_t s,
-                                         uint32_t len, uint32_t t, uint32_t nt) {
+                                         uint32_t len, uint32_t t, uint32_t nt, bool split = false) {
     if (EMIT == kEmitRecord && ep.rp.rec.words <= 8) {
         const fg_record_desc& rec = ep.rp.rec;
         const uint32_t words = rec.words;  // 4 or 8: records are 16-byte aligned
@@ -398,17 +468,11 @@ __device__ __forceinline__ void emit_run(const EmitParams& ep, uint32_t* sperm, 
         // every column a straight copy of [lo, lo + len) to [s, s + len); runs of
         // four 4-byte columns go four rows at a time (16 loads before any store)
         const ColumnParams& cp = ep.cp;
-        if (cp.keep_perm)
+        if (cp.keep_perm || split)
             for (uint32_t k = t; k < len; k += nt) sperm[s + k] = lo + k;
-        for (uint32_t c0 = 0; c0 < cp.ncols; c0 += 4) {
-            const uint32_t nk = min(4u, cp.ncols - c0);
-            bool words = true;
-            for (uint32_t c = 0; c < nk; ++c) words = words && cp.col[c0 + c].elem_bytes == 4u;
-            if (!words) {
-                for (uint32_t c = 0; c < nk; ++c)
-                    for (uint32_t k = t; k < len; k += nt) copy_column_elem(cp.col[c0 + c], lo + k, s + k);
-                continue;
-            }
+        if (split) return;
+        for (uint32_t c0 = 0; c0 < cp.nwords; c0 += 4) {
+            const uint32_t nk = min(4u, cp.nwords - c0);
             for (uint32_t k0 = t; k0 < len; k0 += 4 * nt) {
                 uint32_t v[4][4];
 #pragma unroll
@@ -426,6 +490,17 @@ __device__ __forceinline__ void emit_run(const EmitParams& ep, uint32_t* sperm, 
                         if (c < nk && k < len) static_cast<uint32_t*>(cp.col[c0 + c].out)[s + k] = v[c][m];
                     }
             }
+        }
+        for (uint32_t c = cp.nwords; c < cp.ncols; ++c) {
+            const fg_column& col = cp.col[c];
+            if (col.elem_bytes == 8u)
+                copy_run<uint2>(col, lo, s, len, t, nt);
+            else if (col.elem_bytes == 16u)
+                copy_run<uint4>(col, lo, s, len, t, nt);
+            else if (col.elem_bytes == 1u)
+                copy_run<uint8_t>(col, lo, s, len, t, nt);
+            else
+                for (uint32_t k = t; k < len; k += nt) copy_column_elem(col, lo + k, s + k);
         }
     } else {
         for (uint32_t k = t; k < len; k += nt) emit<EMIT>(ep, sperm, lo + k, s + k);
@@ -450,6 +525,7 @@ struct StabJob {
     const uint32_t* rows;
     uint32_t max_n;
     const uint32_t* slot;
+    uint32_t may_split;  // an agent sort whose columns may be moved by k_gather_columns
 };
 
 __device__ __forceinline__ void queue_long_bin(const StabJob& j, uint32_t b, uint32_t len) {
@@ -477,6 +553,7 @@ __device__ __forceinline__ void stabilize_positions(const StabJob& j, uint32_t b
         emit_run<EMIT>(j.rp, j.sperm, 0u, 0u, total, p, stride);
         return;
     }
+    const bool split = EMIT == kEmitPermColumns && j.may_split && rows_in_no_order(j.h, total);
     for (; p < total; p += stride) {
         const uint32_t i = ahead;
         ahead = p + stride < total ? j.perm[p + stride] : 0u;
@@ -499,7 +576,7 @@ __device__ __forceinline__ void stabilize_positions(const StabJob& j, uint32_t b
         if (len > 1) {
             for (uint32_t q = s; q < e; ++q) dst += (j.perm[q] < i) ? 1u : 0u;
         }
-        emit<EMIT>(j.rp, j.sperm, i, dst);
+        emit<EMIT>(j.rp, j.sperm, i, dst, split);
     }
 }
 
@@ -611,6 +688,8 @@ __device__ __forceinline__ void long_bins(const StabJob& job, LongSmem& sm, uint
     uint32_t& s_lo = sm.lo;
     uint32_t& s_hi = sm.hi;
     const uint32_t nchunks = min(job.h->long_count, job.chunk_cap);
+    const bool split = EMIT == kEmitPermColumns && job.may_split && nchunks &&
+                       rows_in_no_order(job.h, load_count(job.rows, job.max_n));
     // warp pass: bins of up to kWarpBin messages
     {
         const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
@@ -630,7 +709,7 @@ __device__ __forceinline__ void long_bins(const StabJob& job, LongSmem& sm, uint
             lo = __reduce_min_sync(0xFFFFFFFFu, lo);
             hi = __reduce_max_sync(0xFFFFFFFFu, hi);
             if (hi - lo == len - 1u) {  // distinct indices filling [lo, hi]: already ascending from lo
-                emit_run<EMIT>(rp, sperm, lo, s, len, lane, 32u);
+                emit_run<EMIT>(rp, sperm, lo, s, len, lane, 32u, split);
             } else if (hi - lo < kWarpSpanWords * 32u) {
                 const uint32_t words = (hi - lo) / 32u + 1u;
                 for (uint32_t w = lane; w < words; w += 32u) bits[w] = 0u;
@@ -665,7 +744,7 @@ __device__ __forceinline__ void long_bins(const StabJob& job, LongSmem& sm, uint
                 for (uint32_t k = lane; k < len; k += 32u) {
                     const uint32_t i = perm[s + k];
                     const uint32_t d = i - lo;
-                    emit<EMIT>(rp, sperm, i, s + pre[d >> 5] + __popc(bits[d >> 5] & ((1u << (d & 31u)) - 1u)));
+                    emit<EMIT>(rp, sperm, i, s + pre[d >> 5] + __popc(bits[d >> 5] & ((1u << (d & 31u)) - 1u)), split);
                 }
                 __syncwarp();  // bits and pre are reused by the warp's next bin
             } else {
@@ -691,7 +770,7 @@ __device__ __forceinline__ void long_bins(const StabJob& job, LongSmem& sm, uint
                         __syncwarp();
                     }
                 }
-                for (uint32_t k = lane; k < len; k += 32u) emit<EMIT>(rp, sperm, w[k], s + k);
+                for (uint32_t k = lane; k < len; k += 32u) emit<EMIT>(rp, sperm, w[k], s + k, split);
                 __syncwarp();  // w is reused by the warp's next bin
             }
         }
@@ -727,7 +806,7 @@ __device__ __forceinline__ void long_bins(const StabJob& job, LongSmem& sm, uint
             lo = s_lo;
             hi = s_hi;
             if (hi - lo == len - 1u) {  // distinct indices filling [lo, hi]: already ascending from lo
-                emit_run<EMIT>(rp, sperm, lo, s, len, threadIdx.x, blockDim.x);
+                emit_run<EMIT>(rp, sperm, lo, s, len, threadIdx.x, blockDim.x, split);
                 continue;
             }
             if (hi - lo < kSpanCap) {
@@ -758,7 +837,7 @@ __device__ __forceinline__ void long_bins(const StabJob& job, LongSmem& sm, uint
                     const uint32_t i = perm[s + k];
                     const uint32_t d = i - lo;
                     const uint32_t rank = before[d >> 5] + __popc(bits[d >> 5] & ((1u << (d & 31u)) - 1u));
-                    emit<EMIT>(rp, sperm, i, s + rank);
+                    emit<EMIT>(rp, sperm, i, s + rank, split);
                 }
                 continue;
             }
@@ -782,7 +861,7 @@ __device__ __forceinline__ void long_bins(const StabJob& job, LongSmem& sm, uint
                     __syncthreads();
                 }
             }
-            for (uint32_t k = threadIdx.x; k < len; k += blockDim.x) emit<EMIT>(rp, sperm, s_idx[k], s + k);
+            for (uint32_t k = threadIdx.x; k < len; k += blockDim.x) emit<EMIT>(rp, sperm, s_idx[k], s + k, split);
             continue;
         }
         const uint32_t q = s + ch.y * kChunk + threadIdx.x;
@@ -800,7 +879,7 @@ __device__ __forceinline__ void long_bins(const StabJob& job, LongSmem& sm, uint
                 rank += r;
             }
         }
-        if (act) emit<EMIT>(rp, sperm, i, s + rank);
+        if (act) emit<EMIT>(rp, sperm, i, s + rank, split);
     }
 }
 
@@ -835,6 +914,44 @@ __global__ void __launch_bounds__(kThreads) k_long_pair(const __grid_constant__ 
         long_bins<EA>(a, sm, blockIdx.x, ga);
     else
         long_bins<EB>(b, sm, blockIdx.x - ga, gridDim.x - ga);
+}
+
+// Column c moved by the stable permutation, eight rows of a thread in flight.
+template <typename T>
+__device__ __forceinline__ void gather_column(const fg_column& c, const uint32_t* __restrict__ sperm, uint32_t n) {
+    const T* __restrict__ in = static_cast<const T*>(c.in);
+    T* __restrict__ out = static_cast<T*>(c.out);
+    const uint32_t stride = gridDim.x * blockDim.x;
+    for (uint32_t p0 = blockIdx.x * blockDim.x + threadIdx.x; p0 < n; p0 += 8u * stride) {
+        uint32_t i[8];
+        T v[8];
+#pragma unroll
+        for (uint32_t m = 0; m < 8; ++m) i[m] = p0 + m * stride < n ? __ldcs(sperm + p0 + m * stride) : 0u;
+#pragma unroll
+        for (uint32_t m = 0; m < 8; ++m)
+            if (p0 + m * stride < n) v[m] = in[i[m]];
+#pragma unroll
+        for (uint32_t m = 0; m < 8; ++m)
+            if (p0 + m * stride < n) __stcs(out + p0 + m * stride, v[m]);
+    }
+}
+
+__global__ void __launch_bounds__(kThreads) k_gather_columns(const __grid_constant__ ColumnParams cp, uint32_t max_n,
+                                                             const uint32_t* d_n, const uint32_t* sperm,
+                                                             const WsHeader* h) {
+    flamegpu::detail::grid_dependency_enter();
+    const uint32_t n = load_count(d_n, max_n);
+    if (!rows_in_no_order(h, n)) return;  // the stabilising kernels moved the columns
+    for (uint32_t c = 0; c < cp.ncols; ++c) {
+        const fg_column& col = cp.col[c];
+        if (col.elem_bytes == 4u)
+            gather_column<uint32_t>(col, sperm, n);
+        else if (col.elem_bytes == 8u)
+            gather_column<uint2>(col, sperm, n);
+        else
+            for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x)
+                copy_column_elem(col, sperm[p], p);
+    }
 }
 
 // ------------------------------------------------------------------- host side
@@ -903,6 +1020,13 @@ uint32_t grid_for(uint32_t max_n, int per_sm = 8) {
 // covers every chunk of a small list at once; large lists get 4 per SM
 uint32_t long_grid_for(uint32_t max_n) {
     return std::max(1u, std::min((max_n + 127u) / 128u, static_cast<uint32_t>(sm_count() * 4)));
+}
+
+// Whether a sort's columns may be more than L2 holds (see kFarRows).
+bool splits_columns(const fgk::ColumnParams& cp, uint32_t max_n) {
+    uint64_t bytes = 0;
+    for (uint32_t c = 0; c < cp.ncols; ++c) bytes += cp.col[c].elem_bytes;
+    return bytes * max_n > (96ull << 20);
 }
 
 int check_launch() {
@@ -1022,10 +1146,12 @@ int run_pipeline(const fg_spatial_grid* g, const SortGrid& sg, uint32_t nbuckets
     // the scan also compares the keys of rows 32w - 1 and 32w (row order; a batch's keys are never in it)
     const OrderCheck oc{batch.inst ? nullptr : edges, d_n, max_n};
     launch_scan(hist, pbm_out, scan_n, 1, sstat, h, 0, st, key_max, key_floor, oc);
-    launch(k_perm, grid, kThreads, st, PermJob{max_n, d_n, keys, slot, pbm_out, perm, h});
-    const StabJob sj{rp, keys, pbm_out, perm, sperm, chunks, L.chunk_cap, h, key_max, d_n, max_n, slot};
+    const uint32_t may_split = EMIT == kEmitPermColumns && !batch.inst && splits_columns(rp.cp, max_n) ? 1u : 0u;
+    launch(k_perm, grid, kThreads, st, PermJob{max_n, d_n, keys, slot, pbm_out, perm, h, may_split});
+    const StabJob sj{rp, keys, pbm_out, perm, sperm, chunks, L.chunk_cap, h, key_max, d_n, max_n, slot, may_split};
     launch(k_stabilize<EMIT>, grid, kThreads, st, sj);
     launch(k_long<EMIT>, long_grid_for(max_n), kThreads, st, sj);
+    if (may_split) launch(k_gather_columns, grid, kThreads, st, rp.cp, max_n, d_n, static_cast<const uint32_t*>(sperm), static_cast<const WsHeader*>(h));
     return check_launch();
 }
 
@@ -1073,8 +1199,7 @@ int fgi_spatial_sort_agents(const fg_spatial_grid* g, uint32_t max_n, const uint
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     // the stable positions' kernels write every column directly (no gather pass)
     EmitParams rp{};
-    for (uint32_t c = 0; c < ncols; ++c) rp.cp.col[c] = cols[c];
-    rp.cp.ncols = ncols;
+    set_columns(rp.cp, cols, ncols);
     rp.cp.keep_perm = perm_out != nullptr;
     int rc = ncols ? run_pipeline<kSortKey, kEmitPermColumns>(g, sg, nb, max_n, d_n, x, y, z, nullptr, rp,
                                                               reinterpret_cast<uint32_t*>(ws + L.pbm), L, ws, st,
@@ -1119,8 +1244,7 @@ int fgi_spatial_sort_and_build(const fg_spatial_grid* g, uint32_t sort_max_n, co
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     auto at = [](char* w, size_t off) { return reinterpret_cast<uint32_t*>(w + off); };
     EmitParams ea{};
-    for (uint32_t c = 0; c < ncols; ++c) ea.cp.col[c] = cols[c];
-    ea.cp.ncols = ncols;
+    set_columns(ea.cp, cols, ncols);
     ea.cp.keep_perm = 0;
     EmitParams eb{};
     eb.rp.rec = *rec;
@@ -1135,12 +1259,12 @@ int fgi_spatial_sort_and_build(const fg_spatial_grid* g, uint32_t sort_max_n, co
     // each launch gives each sort the blocks its own kernel would have
     const uint32_t ga = grid_for(sort_max_n), gb = grid_for(msg_max_n);
     launch(k_perm_pair, ga + gb, kThreads, st, PermJob{sort_max_n, sort_d_n, at(wa, La.keys), at(wa, La.slot), pbm_a,
-                                                       at(wa, La.perm), ha},
-           PermJob{msg_max_n, msg_d_n, at(wb, Lb.keys), at(wb, Lb.slot), pbm, at(wb, Lb.perm), hb}, ga);
+                                                       at(wa, La.perm), ha, 0u},
+           PermJob{msg_max_n, msg_d_n, at(wb, Lb.keys), at(wb, Lb.slot), pbm, at(wb, Lb.perm), hb, 0u}, ga);
     const StabJob ja{ea, at(wa, La.keys), pbm_a, at(wa, La.perm), at(wa, La.sperm),
-                     reinterpret_cast<uint2*>(wa + La.chunks), La.chunk_cap, ha, &ha->key_max, sort_d_n, sort_max_n, nullptr};
+                     reinterpret_cast<uint2*>(wa + La.chunks), La.chunk_cap, ha, &ha->key_max, sort_d_n, sort_max_n, nullptr, 0u};
     const StabJob jb{eb, at(wb, Lb.keys), pbm, at(wb, Lb.perm), nullptr,
-                     reinterpret_cast<uint2*>(wb + Lb.chunks), Lb.chunk_cap, hb, nullptr, msg_d_n, msg_max_n, at(wb, Lb.slot)};
+                     reinterpret_cast<uint2*>(wb + Lb.chunks), Lb.chunk_cap, hb, nullptr, msg_d_n, msg_max_n, at(wb, Lb.slot), 0u};
     launch(k_stabilize_pair, ga + gb, kThreads, st, ja, jb, ga);
     const uint32_t la = long_grid_for(sort_max_n), lb = long_grid_for(msg_max_n);
     launch(k_long_pair<kEmitPermColumns, kEmitRecord>, la + lb, kThreads, st, ja, jb, la);
@@ -1381,8 +1505,7 @@ extern "C" int fg_spatial_sort_agents_batched(const fg_batch_instance* instances
     char* ws = static_cast<char*>(workspace);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     EmitParams rp{};
-    for (uint32_t c = 0; c < ncols; ++c) rp.cp.col[c] = cols[c];
-    rp.cp.ncols = ncols;
+    set_columns(rp.cp, cols, ncols);
     rp.cp.keep_perm = 0;  // the batched sort returns columns only
     SortGrid sg{};
     BatchKeys bk;

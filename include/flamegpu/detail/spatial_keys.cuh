@@ -59,6 +59,7 @@ __device__ __forceinline__ uint32_t spatial_sort_key(const SortKeyGrid& s, int d
 // Words of a build workspace's header that a key-computing launch resets for
 // the kernels after it (the layout of the kernels' workspace header).
 constexpr int kWsHdrScanEpoch = 1;
+constexpr int kWsHdrFarRows = 2;
 constexpr int kWsHdrLongCount = 4;
 // raised to the largest sort key past the grid's cells (positions outside the
 // environment; 0 if none): the sort's scan stops past max(it, cells - 1)
@@ -88,6 +89,7 @@ constexpr uint32_t kKeyNone = 0, kKeyMessageBin = 1, kKeySortKey = 2;
 // Block 0, thread 0 of the launch: what the key kernel did at its start.
 __device__ __forceinline__ void key_target_reset(const KeyTarget& t) {
     t.header[kWsHdrLongCount] = 0u;
+    t.header[kWsHdrFarRows] = 0u;
     t.header[kWsHdrScanEpoch] = (t.header[kWsHdrScanEpoch] + 1u) & 0x3FFFFFFFu;
 }
 

@@ -1,0 +1,54 @@
+"""Agent sorts whose columns move one after another by the stable permutation
+(more column bytes than L2 holds, rows in no order) and at once (drifted, in
+order, or half of each), through the C ABI against numpy's stable order."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("order", ["random", "half", "drifted", "sorted", "long"])
+@pytest.mark.parametrize("n", [5000, 2_500_000])
+def test_sort_moves_every_column(n, order):
+    import torch
+    from flamegpu2_gb300 import capi
+    L = capi.lib()
+    rng = np.random.default_rng(n + len(order))
+    cells = 8 if order == "long" else max(2, int((n / 3.0) ** (1.0 / 3.0)))
+    pos = rng.uniform(0.0, cells, (n, 3)).astype(np.float32)
+    w = np.float32(cells)
+    cell = lambda p, a: np.floor((p[:, a] / w) * w).astype(np.int64)  # noqa: E731  (the sort key's own float32 arithmetic)
+    key_of = lambda p: (cell(p, 2) * cells + cell(p, 1)) * cells + cell(p, 0)  # noqa: E731
+    if order in ("half", "drifted", "sorted"):
+        pos = pos[np.argsort(key_of(pos), kind="stable")]
+    if order == "drifted":
+        top = np.nextafter(np.float32(cells), np.float32(0))
+        pos = np.clip(pos + rng.normal(0.0, 0.05, pos.shape), 0.0, top).astype(np.float32)
+    if order == "half":
+        pos[:n // 2] = rng.permutation(pos[:n // 2])
+    cols = [np.ascontiguousarray(pos[:, a]) for a in range(3)]
+    cols += [rng.integers(0, 1 << 30, n).astype(np.int32) for _ in range(7)]  # ten 4-byte columns
+    cols += [rng.integers(0, 1 << 60, n) for _ in range(3)]                   # three 8-byte ones
+    cols += [rng.integers(0, 250, n).astype(np.uint8), rng.integers(0, 250, n).astype(np.int16),
+             rng.integers(0, 250, (n, 4)).astype(np.int32), rng.integers(0, 250, (n, 3)).astype(np.int32)]
+    ins = [torch.from_numpy(c).cuda() for c in cols]
+    outs = [torch.zeros_like(c) for c in ins]
+    mixed = rng.permutation(len(ins))  # the order they are given in is free
+    g = capi.grid(3, (0, 0, 0), (cells,) * 3, 1.0)
+    perm = torch.zeros(n, dtype=torch.int32, device="cuda")
+    ws = capi.Workspace(L.fg_spatial_sort_workspace_size(n, C.byref(g)))
+    table = capi.columns([(ins[k], outs[k]) for k in mixed])
+    expect = np.argsort(key_of(pos), kind="stable")
+    for perm_out in (None, perm):
+        for o in outs:
+            o.zero_()
+        capi.check(L.fg_spatial_sort_agents(C.byref(g), n, None, ins[0].data_ptr(), ins[1].data_ptr(), ins[2].data_ptr(), table,
+                                            len(ins), capi.ptr(perm_out), ws.ptr, ws.nbytes, capi.stream_handle()),
+                   "fg_spatial_sort_agents")
+        torch.cuda.synchronize()
+        for c, o in zip(cols, outs):
+            np.testing.assert_array_equal(o.cpu().numpy(), c[expect])
+    np.testing.assert_array_equal(perm.cpu().numpy(), expect)
+    assert ws.status() == 0
