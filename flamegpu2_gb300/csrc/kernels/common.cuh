@@ -97,17 +97,6 @@ __device__ __forceinline__ uint32_t lanemask_lt() {
     return m;
 }
 
-// Warp-aggregated atomicAdd(&hist[key], 1): lanes with equal keys share one
-// atomic; each gets old + its rank among lower lanes with the same key.
-__device__ __forceinline__ uint32_t warp_aggregated_inc(uint32_t* hist, uint32_t key, uint32_t active) {
-    const uint32_t peers = __match_any_sync(active, key);
-    const uint32_t leader = __ffs(peers) - 1;
-    uint32_t base = 0;
-    if (lane_id() == leader) base = atomicAdd(hist + key, static_cast<uint32_t>(__popc(peers)));
-    base = __shfl_sync(peers, base, leader);
-    return base + __popc(peers & lanemask_lt());
-}
-
 inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 }  // namespace fgk

@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(kThreads) k_bin(fg_spatial_grid g, SortGrid sg
                                                   const float* __restrict__ z, const uint32_t* __restrict__ valid,
                                                   uint32_t* __restrict__ keys, uint32_t* __restrict__ slot,
                                                   uint32_t* hist, WsHeader* h, uint32_t pstride,
-                                                  uint32_t* __restrict__ edges) {
+                                                  uint32_t* __restrict__ edges, uint32_t few) {
     flamegpu::detail::grid_dependency_enter();
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         h->long_count = 0;
@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(kThreads) k_bin(fg_spatial_grid g, SortGrid sg
     // with little between them (4,000,037 rows in no order: one row in flight
     // 82 us, four 68 us)
     for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += kBinRows * stride) {
-        uint32_t key[kBinRows], peers[kBinRows], slots[kBinRows];
+        uint32_t key[kBinRows], leader[kBinRows], rank[kBinRows], slots[kBinRows];
 #pragma unroll
         for (int q = 0; q < kBinRows; ++q) {
             const uint32_t i = base + q * stride + threadIdx.x;
@@ -96,13 +96,12 @@ __global__ void __launch_bounds__(kThreads) k_bin(fg_spatial_grid g, SortGrid sg
         }
 #pragma unroll
         for (int q = 0; q < kBinRows; ++q) {
-            const uint32_t m = __ballot_sync(0xFFFFFFFFu, key[q] != kInvalid);
-            peers[q] = 0u;
+            const flamegpu::detail::KeyGroup group(0xFFFFFFFFu, key[q], few != 0u);
+            leader[q] = group.leader;
+            rank[q] = group.rank;
             slots[q] = 0u;
             if (key[q] != kInvalid) {
-                peers[q] = __match_any_sync(m, key[q]);
-                if (lane_id() == static_cast<uint32_t>(__ffs(peers[q]) - 1))
-                    slots[q] = atomicAdd(hist + key[q], static_cast<uint32_t>(__popc(peers[q])));
+                if (lane_id() == group.leader) slots[q] = atomicAdd(hist + key[q], group.len);
                 // the sort's scan stops past the cells, or past the largest key of
                 // a row outside them (rare)
                 if (MODE == kSortKey && key[q] >= cells) atomicMax(&h->key_max, key[q]);
@@ -112,8 +111,7 @@ __global__ void __launch_bounds__(kThreads) k_bin(fg_spatial_grid g, SortGrid sg
         for (int q = 0; q < kBinRows; ++q) {
             const uint32_t i = base + q * stride + threadIdx.x;
             const bool act = i >= base && i < n;
-            if (peers[q])
-                slots[q] = __shfl_sync(peers[q], slots[q], __ffs(peers[q]) - 1) + __popc(peers[q] & lanemask_lt());
+            slots[q] = __shfl_sync(0xFFFFFFFFu, slots[q], leader[q]) + rank[q];
             if (act) {
                 keys[i] = key[q];
                 slot[i] = slots[q];
@@ -154,7 +152,7 @@ __global__ void __launch_bounds__(kThreads) k_bin_batched(const fg_batch_instanc
                                                           const float* __restrict__ y, const float* __restrict__ z,
                                                           const uint32_t* __restrict__ valid,
                                                           uint32_t* __restrict__ keys, uint32_t* __restrict__ slot,
-                                                          uint32_t* hist, WsHeader* h) {
+                                                          uint32_t* hist, WsHeader* h, uint32_t few) {
     flamegpu::detail::grid_dependency_enter();
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         h->long_count = 0;
@@ -195,9 +193,10 @@ __global__ void __launch_bounds__(kThreads) k_bin_batched(const fg_batch_instanc
                 }
             }
         }
-        const uint32_t m = __ballot_sync(0xFFFFFFFFu, key != kInvalid);
+        const flamegpu::detail::KeyGroup group(0xFFFFFFFFu, key, few != 0u);
         uint32_t sl = 0;
-        if (key != kInvalid) sl = warp_aggregated_inc(hist, key & ~kPadBit, m);
+        if (key != kInvalid && lane_id() == group.leader) sl = atomicAdd(hist + (key & ~kPadBit), group.len);
+        sl = __shfl_sync(0xFFFFFFFFu, sl, group.leader) + group.rank;
         if (act) {
             keys[i] = key;
             slot[i] = sl;
@@ -1128,14 +1127,15 @@ int run_pipeline(const fg_spatial_grid* g, const SortGrid& sg, uint32_t nbuckets
     uint2* chunks = reinterpret_cast<uint2*>(ws + L.chunks);
     uint32_t* edges = reinterpret_cast<uint32_t*>(ws + L.edges);
     const uint32_t grid = grid_for(max_n);
+    const uint32_t few = nbuckets <= flamegpu::detail::kFewBuckets ? 1u : 0u;
     if (keys_ready) {
         // the launch before wrote keys, slots and the histogram (key_targets_write)
     } else if (batch.inst) {
         launch(k_bin_batched<MODE>, grid, kThreads, st, batch.inst, batch.counts, batch.ninst, max_n, batch.dims, x, y, z,
-               valid, keys, slot, hist, h);
+               valid, keys, slot, hist, h, few);
     } else {
         launch(k_bin<MODE>, grid, kThreads, st, *g, sg, max_n, d_n, x, y, z, valid, keys, slot, hist, h, pos_stride,
-               edges);
+               edges, few);
     }
     const uint32_t scan_n = nbuckets + 1;
     // an agent sort's buckets (2^bits) run past the grid's cells: its scan stops
@@ -1291,6 +1291,7 @@ int fgi_key_target(const fg_spatial_grid* g, uint32_t max_n, bool sort_mode, voi
     char* ws = static_cast<char*>(workspace);
     t->mode = sort_mode ? flamegpu::detail::kKeySortKey : flamegpu::detail::kKeyMessageBin;
     t->dims = static_cast<uint32_t>(g->dims);
+    t->few = nb <= flamegpu::detail::kFewBuckets ? 1u : 0u;
     t->grid = *g;
     t->keys = reinterpret_cast<uint32_t*>(ws + L.keys);
     t->slot = reinterpret_cast<uint32_t*>(ws + L.slot);

@@ -73,6 +73,7 @@ constexpr int kWsHdrDisorder = 12;
 struct KeyTarget {
     uint32_t mode;           // kKeyNone, kKeyMessageBin or kKeySortKey
     uint32_t dims;
+    uint32_t few;            // at most kFewBuckets buckets
     fg_spatial_grid grid;    // message bins
     SortKeyGrid sort;        // sort keys
     const float* x;          // positions: the message's (by message row) or the agent's (by agent row)
@@ -100,39 +101,69 @@ __device__ __forceinline__ uint32_t key_target_key(const KeyTarget& t, bool vali
                                     : spatial_sort_key(t.sort, static_cast<int>(t.dims), px, py, pz);
 }
 
+/** Lanes of a warp that share one histogram atomic: `leader` adds `len`, and
+ * a lane's place among them is `rank`. Normally they are a run of neighbouring
+ * lanes with equal keys: rows in key order, or drifted from it, have few runs,
+ * and rows in no order over many buckets have hardly a key twice in a warp.
+ * Over few buckets (`few`) the lanes with an equal key anywhere in the warp
+ * share: __match_any_sync finds them, in a pass for each distinct key on the
+ * unit that also serves the constant loads, which it kept busy 72% of the time
+ * in the output launch of 1,048,576 Boids in no order (57.7 us, 46.9 by runs;
+ * a standalone key kernel of 4,000,037 rows 68 and 44 us). */
+struct KeyGroup {
+    uint32_t leader, rank, len;
+    // by the lanes of `active`, which all take part; lanes without a key
+    // (0xFFFFFFFF) form groups of their own
+    __device__ __forceinline__ KeyGroup(uint32_t active, uint32_t key, bool few) {
+        const uint32_t lane = threadIdx.x & 31u;
+        if (few) {  // the same for every lane
+            const uint32_t peers = __match_any_sync(active, key);
+            leader = static_cast<uint32_t>(__ffs(peers) - 1);
+            rank = static_cast<uint32_t>(__popc(peers & ((1u << lane) - 1u)));
+            len = static_cast<uint32_t>(__popc(peers));
+            return;
+        }
+        const uint32_t below = __shfl_up_sync(active, key, 1);
+        const bool head = lane == 0u || !((active >> (lane - 1u)) & 1u) || below != key;
+        const uint32_t heads = __ballot_sync(active, head);
+        leader = 31u - __clz(heads & (0xFFFFFFFFu >> (31u - lane)));
+        rank = lane - leader;
+        // the next head, or the first lane that takes no part, ends the run
+        const uint32_t ends = (heads | ~active) & (0xFFFFFFFEu << lane);
+        len = (ends ? static_cast<uint32_t>(__ffs(ends) - 1) : 32u) - leader;
+    }
+};
+// Buckets up to which the lanes of an equal key anywhere share: a build of
+// 1,000,000 rows in no order over 64 bins took 2,357 us that way and 2,440 by
+// runs; over 512 bins 372 and 370, over 32,768 bins 112 and 111.
+constexpr uint32_t kFewBuckets = 256;
+
 // Histogram counts and slots of the keys k[0], k[1] of rows row[0], row[1]
 // for the targets t[0], t[1] (mode kKeyNone: skipped), by the lanes that
-// reach it together: lanes with the same key share one atomic, and the two
-// targets' atomics are issued before either result is used. Returns bit j set
+// reach it together: lanes with the same key share an atomic (KeyGroup), and the
+// two targets' atomics are issued before either result is used. Returns bit j set
 // where target j's rows here are out of order (the same in every lane); the
 // launch raises the targets' disorder flags once per block at its end
 // (key_targets_order_flush), so a launch over unsorted rows does not store to
 // one word from every warp.
 __device__ __forceinline__ uint32_t key_targets_write(const KeyTarget (&t)[2], const uint32_t (&row)[2],
                                                       const uint32_t (&k)[2]) {
-    // the lanes here together (rows skipped or finished earlier are not);
-    // every one of them executes the ballots, those with a key the matches
+    // the lanes here together (rows skipped or finished earlier are not)
     const uint32_t active = __activemask();
     const uint32_t lane = threadIdx.x & 31u;
-    uint32_t peers[2] = {0u, 0u}, base[2] = {0u, 0u};
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-        if (t[j].mode == kKeyNone) continue;  // the same for every lane
-        const uint32_t counted = __ballot_sync(active, k[j] != 0xFFFFFFFFu);
-        if (k[j] != 0xFFFFFFFFu) peers[j] = __match_any_sync(counted, k[j]);
-    }
+    const KeyGroup group[2] = {KeyGroup(active, k[0], t[0].few != 0u), KeyGroup(active, k[1], t[1].few != 0u)};
+    uint32_t base[2] = {0u, 0u};
 #pragma unroll
     for (int j = 0; j < 2; ++j)
-        if (peers[j] && lane == static_cast<uint32_t>(__ffs(peers[j]) - 1))
-            base[j] = atomicAdd(t[j].hist + k[j], static_cast<uint32_t>(__popc(peers[j])));
+        if (t[j].mode != kKeyNone && k[j] != 0xFFFFFFFFu && lane == group[j].leader)
+            base[j] = atomicAdd(t[j].hist + k[j], group[j].len);
     // an agent sort's scan stops past the grid's cells, or past the largest
     // key of a row outside them (rare: one atomic per such row)
     if (t[1].mode == kKeySortKey && k[1] >= sort_cells(t[1].sort)) atomicMax(t[1].header + kWsHdrKeyMax, k[1]);
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
         if (t[j].mode == kKeyNone) continue;
-        uint32_t s = 0;
-        if (peers[j]) s = __shfl_sync(peers[j], base[j], __ffs(peers[j]) - 1) + __popc(peers[j] & ((1u << lane) - 1u));
+        const uint32_t s = __shfl_sync(active, base[j], group[j].leader) + group[j].rank;
         t[j].keys[row[j]] = k[j];
         t[j].slot[row[j]] = s;
     }

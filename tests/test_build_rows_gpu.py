@@ -47,3 +47,26 @@ def test_build_rows(n, words, drifted, optional):
     np.testing.assert_array_equal(got[:, :3].view(np.float32), pos[order])
     np.testing.assert_array_equal(got[:, 3:3 + words], payload[order])
     assert ws.status() == 0
+
+
+@pytest.mark.parametrize("shuffled", [False, True])
+@pytest.mark.parametrize("cells", [1, 6, 7, 16])  # 216 and 343 bins: at and past the buckets that share by match
+def test_key_groups_in_a_model_and_standalone(cells, shuffled):
+    # a population whose warps hold long runs, single lanes and messages not output
+    from flamegpu2_gb300 import sim
+    n, rng = 5003, np.random.default_rng(cells)
+    pos = rng.uniform(0.0, cells, (n, 3)).astype(np.float32)
+    if not shuffled:
+        key = (pos[:, 2].astype(int) * cells + pos[:, 1].astype(int)) * cells + pos[:, 0].astype(int)
+        pos = pos[np.argsort(key, kind="stable")]
+    out = (rng.random(n) < 0.7).astype(np.int32)
+    s = sim.Simulation("spatial_count", [3, 0, 0, 0, cells, cells, cells, 1.0, 0, 1])
+    s.set_population("agent", n, {"x": pos[:, 0].copy(), "y": pos[:, 1].copy(), "z": pos[:, 2].copy(), "do_output": out})
+    s.step(2)
+    got = np.stack([s.get("agent", k, np.float32) for k in ("x", "y", "z")], 1)
+    counts = np.zeros((cells,) * 3, np.int64)
+    np.add.at(counts, tuple(pos[out == 1].astype(int).T), 1)
+    padded = np.pad(counts, 1)
+    around = sum(padded[a:a + cells, b:b + cells, c:c + cells] for a in range(3) for b in range(3) for c in range(3))
+    np.testing.assert_array_equal(s.get("agent", "count", np.uint32), around[tuple(got.astype(int).T)])
+    s.close()
