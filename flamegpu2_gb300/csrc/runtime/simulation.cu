@@ -283,6 +283,8 @@ struct HostXfer {
     uint32_t* rows_out;        // set: the list's device count (= rows); get: a host word for the count
     uint32_t* max_target;      // set: next id, raised to max_value and past every id of column id_col
     uint32_t max_value;
+    uint32_t* next_target;     // set from device columns: next id, set to next_value
+    uint32_t next_value;
     int32_t id_col;            // set: the id column, checked here (16-byte path only); -1: none
     uint32_t* id_unset;        // set: a host word raised when an id of id_col is unset (0)
     const uint32_t* word_src[kHostXferWords];  // get: status words copied to word_dst
@@ -295,6 +297,11 @@ struct HostXfer {
     unsigned long long* acc;
 };
 
+// whether column c goes in 16-byte pieces
+__device__ __forceinline__ bool xfer_wide(const HostXfer& x, uint32_t c) {
+    return ((reinterpret_cast<uintptr_t>(x.src[c]) | reinterpret_cast<uintptr_t>(x.dst[c])) & 15) == 0;
+}
+
 __global__ void k_host_xfer(const __grid_constant__ HostXfer x) {
     grid_dependency_enter();
     const uint32_t rows = x.d_rows ? min(*x.d_rows, x.rows) : x.rows;
@@ -302,6 +309,7 @@ __global__ void k_host_xfer(const __grid_constant__ HostXfer x) {
     if (tid == 0) {
         if (x.rows_out) *x.rows_out = x.d_rows ? *x.d_rows : rows;
         if (x.max_target && x.max_value) atomicMax(x.max_target, x.max_value);
+        if (x.next_target) *x.next_target = x.next_value;
         if (x.acc) {  // after rows_out: the same thread's store is visible to its loads
             unsigned long long c = 0;
             for (uint32_t k = 0; k < x.ncounts; ++k) c += *x.counts[k];
@@ -321,12 +329,8 @@ __global__ void k_host_xfer(const __grid_constant__ HostXfer x) {
 #pragma unroll
         for (uint32_t j = 0; j < 8; ++j) {
             n16[j] = 0;
-            if (j < nc) {
-                const size_t bytes = static_cast<size_t>(rows) * x.elem_bytes[c0 + j];
-                const uintptr_t a = reinterpret_cast<uintptr_t>(x.src[c0 + j]) | reinterpret_cast<uintptr_t>(x.dst[c0 + j]);
-                if (((a | bytes) & 15) == 0) n16[j] = bytes / 16;
-                most = n16[j] > most ? n16[j] : most;
-            }
+            if (j < nc && xfer_wide(x, c0 + j)) n16[j] = static_cast<size_t>(rows) * x.elem_bytes[c0 + j] / 16;
+            most = n16[j] > most ? n16[j] : most;
         }
         for (size_t k = tid; k < most; k += nthreads) {
             uint4 v[8];
@@ -344,7 +348,24 @@ __global__ void k_host_xfer(const __grid_constant__ HostXfer x) {
                 }
         }
     }
+    // what the 16-byte pieces leave of each column: a byte a thread, all
+    // columns at once. (With the whole of a column of an odd number of rows
+    // copied word by word instead, one column after another, setting 1,021
+    // agents of seven columns took 40 us and reading them 28, now 19 and 21.)
+    for (uint32_t k = tid; k < 16u * x.ncols; k += nthreads) {
+        const uint32_t c = k >> 4, left = k & 15u;
+        if (!xfer_wide(x, c)) continue;
+        const size_t bytes = static_cast<size_t>(rows) * x.elem_bytes[c], at = (bytes & ~static_cast<size_t>(15)) + left;
+        if (at >= bytes) continue;
+        x.dst[c][at] = x.src[c][at];
+        if (static_cast<int32_t>(c) == x.id_col && (left & 3u) == 0u) {
+            const uint32_t id = *reinterpret_cast<const uint32_t*>(x.src[c] + at);
+            id_max = max(id_max, id);
+            id_unset |= id == 0u ? 1u : 0u;
+        }
+    }
     if (x.id_col >= 0) {
+        __syncwarp();
         id_max = __reduce_max_sync(0xFFFFFFFFu, id_max);
         id_unset = __reduce_or_sync(0xFFFFFFFFu, id_unset);
         if ((threadIdx.x & 31u) == 0) {
@@ -352,14 +373,13 @@ __global__ void k_host_xfer(const __grid_constant__ HostXfer x) {
             if (id_unset) *x.id_unset = 1u;
         }
     }
-    // the columns not 16-byte aligned: word or byte copies
+    // the columns whose buffers are not 16-byte aligned: word or byte copies
     for (uint32_t c = 0; c < x.ncols; ++c) {
+        if (xfer_wide(x, c)) continue;  // copied above
         const size_t bytes = static_cast<size_t>(rows) * x.elem_bytes[c];
         const char* s = x.src[c];
         char* d = x.dst[c];
-        if (((reinterpret_cast<uintptr_t>(s) | reinterpret_cast<uintptr_t>(d) | bytes) & 15) == 0) {
-            continue;  // copied above
-        } else if (((reinterpret_cast<uintptr_t>(s) | reinterpret_cast<uintptr_t>(d) | bytes) & 3) == 0) {
+        if (((reinterpret_cast<uintptr_t>(s) | reinterpret_cast<uintptr_t>(d) | bytes) & 3) == 0) {
             const uint32_t* s1 = reinterpret_cast<const uint32_t*>(s);
             uint32_t* d1 = reinterpret_cast<uint32_t*>(d);
             for (size_t k = tid; k < bytes / 4; k += nthreads) d1[k] = s1[k];
@@ -388,6 +408,15 @@ inline void* host_mapped(const void* p) {
         return nullptr;
     }
     return a.type == cudaMemoryTypeHost ? a.devicePointer : nullptr;
+}
+
+inline bool device_memory(const void* p) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeDevice;
 }
 
 // Device buffers of one simulation, taken stream-ordered from the device's
@@ -3053,10 +3082,9 @@ void CUDASimulation::setPopulationColumns(const std::string& agent, const std::s
         mapped = x.src[v] != nullptr;
     }
     // the ids: checked (every one set) and their largest found by the transfer
-    // launch when the id column takes its 16-byte path, else here on the host
+    // launch when the id column goes in 16-byte pieces, else here on the host
     const bool dev_ids = mapped && idc < src.size() && n && impl->h_pinned_dev &&
-                         ((reinterpret_cast<uintptr_t>(x.src[idc]) | reinterpret_cast<uintptr_t>(x.dst[idc]) |
-                           (static_cast<size_t>(n) * sizeof(id_t))) & 15) == 0;
+                         ((reinterpret_cast<uintptr_t>(x.src[idc]) | reinterpret_cast<uintptr_t>(x.dst[idc])) & 15) == 0;
     id_t mx = 0;
     if (idc < src.size() && n && !dev_ids) {
         // one branch-free pass (it vectorises): the largest id, and whether any is unset
@@ -3316,12 +3344,52 @@ void CUDASimulation::setPopulationDevice(const std::string& agent, const std::st
     detail::AgentList* l = impl->list_of(agent, state);
     if (columns.size() != l->cols.size())
         THROW exception::InvalidArgument(format("setPopulationDevice needs all %zu variables of agent '%s'", l->cols.size(), agent.c_str()));
-    FG_CUDA(cudaStreamSynchronize(impl->stream));
-    if (n > l->capacity) impl->ensure_capacity(*l, n, 0);
+    // only growing the buffers needs the stream idle (the copies are ordered after its earlier work)
+    if (n > l->capacity) {
+        FG_CUDA(cudaStreamSynchronize(impl->stream));
+        impl->ensure_capacity(*l, n, 0);
+    }
     impl->ensure_all_allocated();
+    detail::HostXfer x;
+    std::memset(&x, 0, sizeof(x));
+    x.id_col = -1;
+    size_t total = 0;
+    bool one_launch = columns.size() <= static_cast<size_t>(detail::kHostXferCols);
     for (const auto& c : columns) {
         const int v = l->var_index(c.first);
         if (v < 0) THROW exception::InvalidAgentVar(format("Agent '%s' has no variable '%s'", agent.c_str(), c.first.c_str()));
+        if (!one_launch) continue;
+        x.src[x.ncols] = static_cast<const char*>(c.second);
+        x.dst[x.ncols] = static_cast<char*>(l->cols[v][l->parity]);
+        x.elem_bytes[x.ncols] = l->agent->variables[v].bytes();
+        total += static_cast<size_t>(n) * x.elem_bytes[x.ncols];
+        one_launch = (reinterpret_cast<uintptr_t>(c.second) & 15) == 0 && (n == 0 || detail::device_memory(c.second));
+        ++x.ncols;
+    }
+    // up to 64 MB of aligned device columns: one launch copies them all and
+    // sets the count, the next id and the recount, instead of a copy each, two
+    // more for the words and a second wait (100,003 Boids 55 us, 31 us so);
+    // larger populations take the copies, which move more bytes a second
+    if (one_launch && total <= (64u << 20)) {
+        x.rows = n;
+        x.rows_out = l->d_count;
+        x.next_target = impl->d_next_id(impl->agent_index(l->agent));
+        x.next_value = next_id;
+        detail::StepEnd e{};
+        impl->count_targets(e);
+        for (uint32_t k = 0; k < e.ncounts; ++k) x.counts[k] = e.counts[k];
+        x.ncounts = e.ncounts;
+        x.acc = e.acc;
+        FG_CUDA(detail::launch_kernel(detail::pdl_enabled(), detail::k_host_xfer, detail::host_xfer_grid(x, impl->sms), 256, 0,
+                                      impl->stream, x));
+        l->bound = n;
+        impl->forget_counts(true);
+        FG_CUDA(cudaStreamSynchronize(impl->stream));
+        return;
+    }
+    FG_CUDA(cudaStreamSynchronize(impl->stream));  // h_pinned's words may be in use by an earlier call's copies
+    for (const auto& c : columns) {
+        const int v = l->var_index(c.first);
         const size_t b = l->agent->variables[v].bytes();
         if (n) FG_CUDA(cudaMemcpyAsync(l->cols[v][l->parity], c.second, b * n, cudaMemcpyDeviceToDevice, impl->stream));
     }
