@@ -107,13 +107,58 @@ constexpr uint32_t kRowAlign = kAgentBlock;
 
 uint32_t round_rows(uint32_t n) { return std::max(kRowAlign, (n + kRowAlign - 1) / kRowAlign * kRowAlign); }
 
+// One run's values of one variable, on their way between its AgentVector and
+// the batch's column.
+struct Segment {
+    const char* src;
+    char* dst;
+    unsigned long long bytes;
+};
+
+/**
+ * Moves every segment in one launch; src or dst, and the table itself, are
+ * ordinary host memory, which this kernel reads and writes in place over the
+ * chip-to-chip link (the device uses the host's page tables).
+ *
+ * Bound by that link. A copy call per run and variable costs its 9.5 us
+ * whatever it moves: 24 runs of 7 variables, 12 MB, 1.6 ms each way; one copy
+ * per variable would need the runs packed together first, 0.8 ms of it. This
+ * launch: 0.11 ms in, 0.13 ms out. With the buffers from the pool (Alloc) 100
+ * steps of those runs take 15.8 ms instead of 21.0, populations in and results
+ * out; 200 runs of 33 million agents spend 73 ms outside their steps instead of 88.
+ */
+constexpr uint32_t kMoveThreads = 256;
+__global__ void __launch_bounds__(kMoveThreads) k_move_segments(const Segment* segs, uint32_t parts) {
+    const Segment s = segs[blockIdx.x / parts];
+    const uint32_t thread = (blockIdx.x % parts) * kMoveThreads + threadIdx.x, threads = parts * kMoveThreads;
+    // both ends on 16 bytes (a vector's storage; a column at a row that is a multiple of the agent block)
+    const unsigned long long n = s.bytes / 16, done = n * 16;
+    const uint4* src = reinterpret_cast<const uint4*>(s.src);
+    uint4* dst = reinterpret_cast<uint4*>(s.dst);
+    unsigned long long i = thread;
+    for (; i + 3ull * threads < n; i += 4ull * threads) {
+        uint4 v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[j] = src[i + static_cast<unsigned long long>(j) * threads];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) dst[i + static_cast<unsigned long long>(j) * threads] = v[j];
+    }
+    for (; i < n; i += threads) dst[i] = src[i];
+    if (done + thread < s.bytes) s.dst[done + thread] = s.src[done + thread];
+}
+
+// Device memory of one batch, zeroed. From the device's stream-ordered pool,
+// on the legacy stream: fourteen buffers of 1.7 MB cost 0.16 ms to get and give
+// back, 1.05 ms as separate allocations, and an ensemble has about thirty. The
+// pool keeps nothing past a synchronisation (its release threshold is the
+// default, 0).
 struct Alloc {
     std::vector<void*> ptrs;
     void* get(size_t bytes) {
         void* p = nullptr;
-        FG_ECUDA(cudaMalloc(&p, std::max<size_t>(bytes, 256)));
-        FG_ECUDA(cudaMemset(p, 0, std::max<size_t>(bytes, 256)));
+        FG_ECUDA(cudaMallocAsync(&p, std::max<size_t>(bytes, 256), cudaStreamLegacy));
         ptrs.push_back(p);
+        FG_ECUDA(cudaMemsetAsync(p, 0, std::max<size_t>(bytes, 256), cudaStreamLegacy));
         return p;
     }
     // frees p (null: nothing); the device must be done with it
@@ -121,7 +166,7 @@ struct Alloc {
         if (!p) return;
         auto it = std::find(ptrs.begin(), ptrs.end(), p);
         if (it != ptrs.end()) {
-            cudaFree(p);
+            cudaFreeAsync(p, cudaStreamLegacy);
             ptrs.erase(it);
         }
     }
@@ -130,7 +175,9 @@ struct Alloc {
         return get(bytes);
     }
     ~Alloc() {
-        for (void* p : ptrs) cudaFree(p);
+        if (ptrs.empty()) return;
+        for (void* p : ptrs) cudaFreeAsync(p, cudaStreamLegacy);
+        cudaStreamSynchronize(cudaStreamLegacy);
     }
 };
 
@@ -267,6 +314,9 @@ struct BatchedSim {
     BatchedSim(std::shared_ptr<ModelData> m, const RunPlanVector& p, const CUDAEnsemble::EnsembleConfig& c)
         : model(std::move(m)), plans(p), cfg(c) {}
     ~BatchedSim() {
+        // the buffers go back in the legacy stream's order, which does not wait for these
+        if (stream) cudaStreamSynchronize(stream);
+        if (side) cudaStreamSynchronize(side);
         drop_graphs();
         for (auto& r : reports)
             if (r.ev) cudaEventDestroy(r.ev);
@@ -348,6 +398,8 @@ struct BatchedSim {
             cols[v] = {mem.get(b * total_rows), mem.get(b * total_rows)};
         }
         std::vector<id_t> next(ninst, 1);
+        std::vector<Segment> segs;
+        std::vector<std::vector<id_t>> kept;  // filled ids, until they are moved
         for (uint32_t k = 0; k < ninst; ++k) {
             auto it = plans[k].populations().find({agent->name, state});
             if (it == plans[k].populations().end() || count[k] == 0) continue;
@@ -367,10 +419,12 @@ struct BatchedSim {
                 const size_t b = agent->variables[v].bytes();
                 const void* src = (v == idc && !filled.empty()) ? static_cast<const void*>(filled.data())
                                                                  : static_cast<const void*>(pop.columns()[v].data());
-                FG_ECUDA(cudaMemcpy(static_cast<char*>(cols[v][0]) + b * row_begin[k], src, b * count[k],
-                                    cudaMemcpyHostToDevice));
+                segs.push_back({static_cast<const char*>(src), static_cast<char*>(cols[v][0]) + b * row_begin[k],
+                                static_cast<unsigned long long>(b) * count[k]});
             }
+            if (!filled.empty()) kept.push_back(std::move(filled));
         }
+        move_segments(segs, cudaMemcpyHostToDevice);
         d_counts = static_cast<uint32_t*>(mem.get(sizeof(uint32_t) * ninst));
         FG_ECUDA(cudaMemcpy(d_counts, count.data(), sizeof(uint32_t) * ninst, cudaMemcpyHostToDevice));
         d_next_ids = static_cast<uint32_t*>(mem.get(sizeof(uint32_t) * ninst));
@@ -560,6 +614,7 @@ struct BatchedSim {
             comp_ws_bytes = fg_compact_batched_workspace_size(comp_tiles, ninst);
             comp_ws = mem.get(comp_ws_bytes);
         }
+        FG_ECUDA(cudaStreamSynchronize(cudaStreamLegacy));  // the buffers' zeros, before any step
         drop_graphs();
     }
     fg_batch_instance* comp_inst = nullptr;  // row segments, for the segmented compaction
@@ -626,6 +681,7 @@ struct BatchedSim {
             const size_t b = agent->variables[v].bytes();
             void* n0 = mem.get(b * total_rows);
             void* n1 = mem.get(b * total_rows);
+            FG_ECUDA(cudaStreamSynchronize(cudaStreamLegacy));  // the zeros, before the rows
             for (uint32_t k = 0; k < ninst; ++k)
                 if (count[k])
                     FG_ECUDA(cudaMemcpyAsync(static_cast<char*>(n0) + b * row_begin[k],
@@ -844,16 +900,46 @@ struct BatchedSim {
 
     double step_seconds = 0.0;  // device time from the first step's start to the last step's end
 
-    AgentVector read_instance(uint32_t k) {
-        AgentVector pop(AgentDescription(model, agent), 0);
-        pop.setCountRaw(count[k]);
-        for (size_t v = 0; v < cols.size(); ++v) {
-            const size_t b = agent->variables[v].bytes();
-            if (count[k])
-                FG_ECUDA(cudaMemcpy(pop.columns()[v].data(), static_cast<char*>(cols[v][parity]) + b * row_begin[k],
-                                    b * count[k], cudaMemcpyDeviceToHost));
+    // Copies the segments, whose host side is ordinary memory of this process;
+    // they are in place on return. The kernel where the device reaches such
+    // memory by the host's page tables, else a copy each.
+    void move_segments(const std::vector<Segment>& segs, cudaMemcpyKind kind) {
+        if (segs.empty()) return;
+        int in_place = 0;
+        cudaDeviceGetAttribute(&in_place, cudaDevAttrPageableMemoryAccessUsesHostPageTables, cfg.device);
+        for (const Segment& s : segs)
+            if ((reinterpret_cast<uintptr_t>(s.src) | reinterpret_cast<uintptr_t>(s.dst)) & 15u) in_place = 0;
+        if (!in_place) {
+            for (const Segment& s : segs) FG_ECUDA(cudaMemcpy(s.dst, s.src, s.bytes, kind));
+            return;
         }
-        return pop;
+        FG_ECUDA(cudaStreamSynchronize(cudaStreamLegacy));  // the columns' zeros
+        // blocks per segment: its 16-byte pieces, four a thread, to eight blocks an SM over all of them
+        unsigned long long most = 0;
+        for (const Segment& s : segs) most = std::max(most, s.bytes);
+        const uint64_t room = std::max<uint64_t>(1, static_cast<uint64_t>(sms) * 8 / segs.size());
+        const uint64_t useful = std::max<uint64_t>(1, (most + kMoveThreads * 64ull - 1) / (kMoveThreads * 64ull));
+        const uint32_t parts = static_cast<uint32_t>(std::min(room, useful));
+        k_move_segments<<<static_cast<unsigned int>(segs.size() * parts), kMoveThreads, 0, stream>>>(segs.data(), parts);
+        FG_ECUDA(cudaGetLastError());
+        FG_ECUDA(cudaStreamSynchronize(stream));
+    }
+
+    // The populations of the runs for which take(k) holds, at their counts.
+    template <typename Take>
+    void read_instances(std::vector<std::shared_ptr<AgentVector>>& results, Take take) {
+        std::vector<Segment> segs;
+        for (uint32_t k = 0; k < ninst; ++k) {
+            if (!take(k)) continue;
+            results[k] = std::make_shared<AgentVector>(AgentDescription(model, agent), 0);
+            results[k]->setCountRaw(count[k]);
+            for (size_t v = 0; count[k] && v < cols.size(); ++v) {
+                const size_t b = agent->variables[v].bytes();
+                segs.push_back({static_cast<char*>(cols[v][parity]) + b * row_begin[k], results[k]->columns()[v].data(),
+                                static_cast<unsigned long long>(b) * count[k]});
+            }
+        }
+        move_segments(segs, cudaMemcpyDeviceToHost);
     }
 
     // One step: captured (or replayed) as a graph per buffer parity and sort decision.
@@ -1104,9 +1190,9 @@ struct BatchedSim {
             if (any) {
                 FG_ECUDA(cudaStreamSynchronize(stream));
                 if (death_or_birth) FG_ECUDA(cudaMemcpy(count.data(), d_counts, sizeof(uint32_t) * ninst, cudaMemcpyDeviceToHost));
+                read_instances(results, [&](uint32_t k) { return plans[k].getSteps() == s + 1; });
                 for (uint32_t k = 0; k < ninst; ++k) {
-                    if (plans[k].getSteps() != s + 1 || s + 1 >= max_steps) continue;
-                    results[k] = std::make_shared<AgentVector>(read_instance(k));
+                    if (plans[k].getSteps() != s + 1) continue;
                     count[k] = 0;
                     bound[k] = 0;
                     FG_ECUDA(cudaMemcpy(d_counts + k, &count[k], sizeof(uint32_t), cudaMemcpyHostToDevice));
@@ -1130,8 +1216,7 @@ struct BatchedSim {
             if (st) THROW exception::DeviceError(format("Batched compaction reported status %d", static_cast<int>(st)));
             FG_ECUDA(cudaMemcpy(count.data(), d_counts, sizeof(uint32_t) * ninst, cudaMemcpyDeviceToHost));
         }
-        for (uint32_t k = 0; k < ninst; ++k)
-            if (!results[k]) results[k] = std::make_shared<AgentVector>(read_instance(k));
+        read_instances(results, [&](uint32_t k) { return !results[k]; });
     }
 };
 
