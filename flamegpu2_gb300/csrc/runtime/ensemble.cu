@@ -21,6 +21,7 @@
 #include <cstring>
 #include <map>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -124,7 +125,7 @@ struct Segment {
  * whatever it moves: 24 runs of 7 variables, 12 MB, 1.6 ms each way; one copy
  * per variable would need the runs packed together first, 0.8 ms of it. This
  * launch: 0.11 ms in, 0.13 ms out. With the buffers from the pool (Alloc) 100
- * steps of those runs take 15.8 ms instead of 21.0, populations in and results
+ * steps of those runs take 16.2 ms instead of 21.0, populations in and results
  * out; 200 runs of 33 million agents spend 73 ms outside their steps instead of 88.
  */
 constexpr uint32_t kMoveThreads = 256;
@@ -147,18 +148,38 @@ __global__ void __launch_bounds__(kMoveThreads) k_move_segments(const Segment* s
     if (done + thread < s.bytes) s.dst[done + thread] = s.src[done + thread];
 }
 
-// Device memory of one batch, zeroed. From the device's stream-ordered pool,
-// on the legacy stream: fourteen buffers of 1.7 MB cost 0.16 ms to get and give
-// back, 1.05 ms as separate allocations, and an ensemble has about thirty. The
-// pool keeps nothing past a synchronisation (its release threshold is the
-// default, 0).
+// Device memory of one batch, zeroed, from a stream-ordered pool of the
+// ensembles' own, on the legacy stream: fourteen buffers of 1.7 MB take 0.16 ms
+// to get (separate allocations: 0.57 ms), an ensemble's thirty or so 0.2 ms to
+// give back (fourteen separate ones: 0.48 ms). Unlike the pool of the
+// simulations, whose freed blocks wait for the next one, this one keeps nothing
+// past a synchronisation (release threshold 0): a batch may be most of the
+// device's memory.
 struct Alloc {
     std::vector<void*> ptrs;
+    static cudaMemPool_t pool() {
+        constexpr int kDevices = 64;
+        static std::mutex lock;
+        static cudaMemPool_t pools[kDevices] = {};
+        int device = 0;
+        FG_ECUDA(cudaGetDevice(&device));
+        if (device < 0 || device >= kDevices) THROW exception::InvalidArgument("Device index out of range");
+        std::lock_guard<std::mutex> g(lock);
+        if (!pools[device]) {
+            cudaMemPoolProps props{};
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = device;
+            FG_ECUDA(cudaMemPoolCreate(&pools[device], &props));
+        }
+        return pools[device];
+    }
     void* get(size_t bytes) {
         void* p = nullptr;
-        FG_ECUDA(cudaMallocAsync(&p, std::max<size_t>(bytes, 256), cudaStreamLegacy));
+        const size_t n = std::max<size_t>(bytes, 256);
+        FG_ECUDA(cudaMallocFromPoolAsync(&p, n, pool(), cudaStreamLegacy));
         ptrs.push_back(p);
-        FG_ECUDA(cudaMemsetAsync(p, 0, std::max<size_t>(bytes, 256), cudaStreamLegacy));
+        FG_ECUDA(cudaMemsetAsync(p, 0, n, cudaStreamLegacy));
         return p;
     }
     // frees p (null: nothing); the device must be done with it
@@ -409,8 +430,14 @@ struct BatchedSim {
             const size_t idc = pop.columnIndex("_id");
             const id_t* ids = reinterpret_cast<const id_t*>(pop.columns()[idc].data());
             std::vector<id_t> filled;
-            for (uint32_t i = 0; i < count[k]; ++i) next[k] = std::max<id_t>(next[k], ids[i] + 1);
+            id_t past = next[k];
+            uint32_t unset = 0;
             for (uint32_t i = 0; i < count[k]; ++i) {
+                past = std::max<id_t>(past, ids[i] + 1);
+                unset |= ids[i] == ID_NOT_SET ? 1u : 0u;
+            }
+            next[k] = past;
+            for (uint32_t i = 0; unset && i < count[k]; ++i) {
                 if (ids[i] != ID_NOT_SET) continue;
                 if (filled.empty()) filled.assign(ids, ids + count[k]);
                 filled[i] = next[k]++;

@@ -231,7 +231,7 @@ int fg_exclusive_scan_u32(const uint32_t* in, uint32_t* out, uint32_t n,
  * memory, one per device; nothing is allocated, now or later. Its limit:
  * n > FG_NOALLOC_SCAN_MAX_N returns FG_ERR_WORKSPACE and launches nothing.
  * The first call on a device, with that device current, does the set-up: it
- * looks up the array's address and clears it (the scan's tile ticket, epoch
+ * looks up the array's address and clears it (the scan's epoch, order flag
  * and tile statuses must start at zero), waiting for that clear to finish.
  * Make that first call before any stream capture. Every later call only
  * launches the scan on `stream` and leaves the scratch ready for the next.

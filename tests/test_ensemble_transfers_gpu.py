@@ -31,3 +31,23 @@ def test_runs_without_steps_return_their_populations(sizes, ids):
             want = pop["_id"] if ids else np.arange(1, n + 1, dtype=np.uint32)
             np.testing.assert_array_equal(ens.get(r, "Boid", "_id", np.uint32), want)
     ens.close()
+
+
+def test_an_ensemble_gives_its_memory_back():
+    import torch
+    from flamegpu2_gb300 import sim, synth
+    params = synth.boids_params(dict(synth.BOIDS_SMALL))
+    s = sim.Simulation("boids_spatial3d", params)  # simulations keep freed blocks in their pool
+    s.set_population("Boid", 1000, synth.boids_population(1000, 0.0, 64.0, 1))
+    s.step(1)
+    s.close()
+
+    def free_after(n):
+        ens = sim.Ensemble("boids_spatial3d", params)
+        ens.add_run(0, 1, "Boid", n, {k: np.zeros(n, np.float32) for k in NAMES})
+        assert ens.simulate() == 0 and ens.stats()["batched"]
+        ens.close()
+        torch.cuda.synchronize()
+        return torch.cuda.mem_get_info()[0]
+    before = free_after(1000)
+    assert free_after(4_000_000) >= before - (64 << 20)  # its columns alone are 224 MB
