@@ -191,9 +191,7 @@ extern "C" int fgs_get_population(fgs_sim* s, const char* agent, const char* sta
 extern "C" int fgs_get_variable_device(fgs_sim* s, const char* agent, const char* state, const char* var, void* dst,
                                        size_t bytes) {
     return guarded([&] {
-        void* src = s->sim->getDeviceVariable(agent, var, state);
-        if (cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, s->sim->getStream()) != cudaSuccess)
-            throw flamegpu::exception::CUDAError("device copy failed");
+        s->sim->getVariableDevice(agent, var, state, dst, bytes);
     });
 }
 

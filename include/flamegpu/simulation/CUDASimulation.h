@@ -488,6 +488,9 @@ class CUDASimulation {
     unsigned int getAgentCount(const std::string& agent, const std::string& state = "default");
     /** Device pointer to the current column of an agent variable (valid until the next step). */
     void* getDeviceVariable(const std::string& agent, const std::string& variable, const std::string& state = "default");
+    /** Copies the first `bytes` of that column to device memory at dst, on the simulation's stream. */
+    void getVariableDevice(const std::string& agent, const std::string& variable, const std::string& state, void* dst,
+                           size_t bytes);
     /** One reduction of an agent variable over its population, on the device
      *  (the step / exit logs' reductions; HostAgentAPI's sum, min, max and
      *  mean / standard deviation use it). GB300 extension. */

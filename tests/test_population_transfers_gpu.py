@@ -82,3 +82,22 @@ def test_device_population_gives_births_the_next_ids():
         np.testing.assert_array_equal(ids, np.concatenate([cols["_id"], next_id + np.arange(n, dtype=np.uint32)]))
         assert s.agent_steps() > 0
     s.close()
+
+
+@pytest.mark.parametrize("n", [1, 3, 4, 5, 1023, 4096, 4097, 700_001, 6_000_001])
+def test_columns_copied_to_device_tensors(n):
+    """Sizes around a piece, a thread's round and a grid's; a tensor at an odd address; part of a column."""
+    import torch
+    from flamegpu2_gb300 import sim
+    s = sim.Simulation("boids_spatial3d")
+    cols = _columns("Boid", n, 3)
+    s.set_population("Boid", n, cols)
+    for k, offset, m in (("x", 0, n), ("fz", 1, n), ("_id", 4, n), ("y", 0, (n + 1) // 2)):
+        buf = torch.full((n + 8,), -1, dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        s.get_device("Boid", k, buf[offset:offset + m])
+        s.synchronize()
+        got = buf.cpu().numpy()
+        np.testing.assert_array_equal(got[offset:offset + m].view(cols[k].dtype), cols[k][:m])
+        assert (got[:offset] == -1).all() and (got[offset + m:] == -1).all()
+    s.close()
