@@ -319,9 +319,11 @@ __global__ void __launch_bounds__(kThreads) k_compact(const __grid_constant__ Co
         }
         __syncthreads();  // s_tile and sm are reused by the next tile
     }
-    // the last block to finish publishes the new count and resets the tickets
-    // (every block counts: until all have read them, the list's count and next
-    // id stay; the ticket is reset once no block will take another)
+    // the last block to finish publishes the new count, flips the parity and
+    // resets the tickets. A block counts as done once all its warps have read
+    // the list's count, next id and the parity: the barrier, which a block past
+    // the population's tiles (it skips the loop) has not met before
+    __syncthreads();
     if (tid == 0) {
         if (atomicAdd(&h->comp_done, 1u) == gridDim.x - 1) {
             __threadfence();

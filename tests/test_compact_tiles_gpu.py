@@ -52,3 +52,37 @@ def test_compaction_tiles(n, p_born, room, layout):
         if c == ncols - 1:
             kid[~kept] = ids[~kept].view(np.uint8).reshape(-1, 4)
         np.testing.assert_array_equal(outs[c].cpu().numpy()[:total], np.concatenate([rows[c][surv], kid])[:cap])
+
+
+@pytest.mark.parametrize("n,spare", [(1, 1), (1024, 1), (5_000, 3), (5_000, 600), (100_000, 90)])
+def test_population_tiles_below_its_capacity(n, spare):
+    """Calls in a row on one workspace, as a simulation makes them (the count in place, both status arrays in turn),
+    with blocks past the population's tiles: they read the count and the parity that the last block then changes."""
+    import torch
+    from flamegpu2_gb300 import capi
+    L = capi.lib()
+    cap = n + spare * 1024
+    rng = np.random.default_rng(n + spare)
+    value = np.arange(n, dtype=np.int32)
+    cols = [torch.zeros(cap, dtype=torch.int32, device="cuda") for _ in range(2)]
+    cols[0][:n] = torch.from_numpy(value).cuda()
+    births = torch.full((cap,), -7, dtype=torch.int32, device="cuda")
+    d_n = torch.tensor([n], dtype=torch.int32, device="cuda")
+    ws = capi.Workspace(L.fg_compact_workspace_size(cap))
+    flags, expect = [], value
+    for _ in range(24):
+        alive, born = (rng.random(cap) < 0.9).astype(np.int32), (rng.random(cap) < 0.1).astype(np.int32)
+        m = len(expect)
+        expect = np.concatenate([expect[alive[:m] == 1], np.full(born[:m].sum(), -7, np.int32)])
+        flags.append((torch.from_numpy(alive).cuda(), torch.from_numpy(born).cuda()))
+        assert len(expect) <= cap
+    torch.cuda.synchronize()
+    for k, (alive, born) in enumerate(flags):  # nothing waits between the calls
+        a, b = cols[k % 2], cols[1 - k % 2]
+        capi.check(L.fg_compact_agents(cap, d_n.data_ptr(), alive.data_ptr(), born.data_ptr(), capi.columns([(a, b)]),
+                                       capi.columns([(births, b)]), 1, -1, None, None, d_n.data_ptr(), cap, ws.ptr,
+                                       ws.nbytes, capi.stream_handle()), "fg_compact_agents")
+    torch.cuda.synchronize()
+    assert ws.status() == 0
+    assert int(d_n.item()) == len(expect)
+    np.testing.assert_array_equal(cols[0].cpu().numpy()[:len(expect)], expect)
