@@ -78,7 +78,8 @@ __device__ __forceinline__ void fill_ctx(const LaunchParams& P, uint32_t base) {
 template <typename F, int MINB, bool BATCH, bool STAGE>
 __global__ void __launch_bounds__(kAgentBlock, MINB) agent_function_kernel(const __grid_constant__ LaunchParams P) {
     grid_dependency_enter();
-    const Launch L{P, BATCH, STAGE};
+    bool words_held = false;
+    const Launch L{P, BATCH, STAGE, words_held};
     using MsgIn = typename F::MessageIn;
     using MsgOut = typename F::MessageOut;
     // rows to visit: the population (single) or every row of the batch
@@ -184,7 +185,8 @@ template <typename C>
 __global__ void __launch_bounds__(kAgentBlock) agent_condition_kernel(const __grid_constant__ LaunchParams P) {
     grid_dependency_enter();
     const uint32_t n = P.d_n ? min(*P.d_n, P.max_n) : P.max_n;
-    const Launch L{P, false, false};
+    bool words_held = false;
+    const Launch L{P, false, false, words_held};
     for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx <= P.max_n; idx += gridDim.x * blockDim.x) {
         uint32_t fail = 0u;
         if (idx < n) {

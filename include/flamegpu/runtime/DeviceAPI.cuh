@@ -62,6 +62,7 @@ struct Launch {
     const LaunchParams& P;
     bool batch;  // ctx() holds the instance of the block's rows
     bool stage;  // the block may have a staged window
+    bool& words_held;  // a wrapped search of this thread holds its range words (a local of the kernel)
     __device__ __forceinline__ operator const LaunchParams&() const { return P; }
     __device__ __forceinline__ const fg_spatial_grid& grid() const { return batch ? ctx().grid : P.in_grid; }
     __device__ __forceinline__ const uint32_t* pbm() const { return batch ? ctx().pbm : P.in_pbm; }
@@ -983,7 +984,7 @@ class StripCursor {
  public:
     // a search keeps nothing but its origin: every walk reads the bounds itself
     struct Shared {
-        __device__ __forceinline__ Shared(const detail::Launch&, const Window&, bool&, const float (&)[3]) {}
+        __device__ __forceinline__ Shared(const detail::Launch&, const Window&, const float (&)[3]) {}
     };
     __device__ __forceinline__ StripCursor(const detail::Launch& l, const Window& w, const Shared&, const float (&p)[3])
         : L(l), win(w) {
@@ -1076,15 +1077,16 @@ class CellCursor {
     }
 
  public:
-    // holds the thread's words while it lives
+    // holds the thread's words while it lives. The words are the thread's, so
+    // the flag is too: every copy of the input list comes to the same one
     struct Shared {
-        bool& busy;
+        bool& held;
         const bool owner;
         bool listed = false;
-        __device__ __forceinline__ Shared(const detail::Launch& L, const Window& win, bool& in_use, const float (&p)[3])
-            : busy(in_use), owner(!in_use) {
+        __device__ __forceinline__ Shared(const detail::Launch& L, const Window& win, const float (&p)[3])
+            : held(L.words_held), owner(!L.words_held) {
             if (!owner) return;
-            busy = true;
+            held = true;
             const Terms terms(L, p);
             uint32_t* w = column();
             const uint32_t bits = L.P.in_index_bits, base = L.row_base();
@@ -1100,9 +1102,9 @@ class CellCursor {
             }
             w[0] = w[detail::kAgentBlock] = 0u;
         }
-        __device__ __forceinline__ Shared(const Shared& o) : busy(o.busy), owner(false) {}
+        __device__ __forceinline__ Shared(const Shared& o) : held(o.held), owner(false) {}
         __device__ __forceinline__ ~Shared() {
-            if (owner) busy = false;
+            if (owner) held = false;
         }
     };
     __device__ __forceinline__ CellCursor(const detail::Launch& l, const Window& w, const Shared& s, const float (&p)[3])
@@ -1172,8 +1174,8 @@ class Search {
         uint32_t end_;
     };
 
-    __device__ __forceinline__ Search(const detail::Launch& l, bool& in_use, float x, float y, float z)
-        : L(l), win(l), loc{x, y, z}, shared(l, win, in_use, loc) {}
+    __device__ __forceinline__ Search(const detail::Launch& l, float x, float y, float z)
+        : L(l), win(l), loc{x, y, z}, shared(l, win, loc) {}
     __device__ __forceinline__ iterator begin() const { return iterator(*this, false); }
     __device__ __forceinline__ iterator end() const { return iterator(*this, true); }
 
@@ -1243,7 +1245,6 @@ class SpatialIn {
     }
     const detail::Launch L;
     const detail::LaunchParams& P;
-    mutable bool busy = false;  // a filter of this thread holds its range words
 };
 
 /** MessageSpatial2D (include/flamegpu/runtime/messaging/MessageSpatial2D/MessageSpatial2DDevice.cuh). */
@@ -1253,10 +1254,10 @@ class MessageSpatial2D {
     class In : public SpatialIn<2> {
      public:
         __device__ explicit In(const detail::Launch& l) : SpatialIn<2>(l) {}
-        __device__ Filter operator()(float x, float y) const { return Filter(L, busy, x, y, 0.0f); }
+        __device__ Filter operator()(float x, float y) const { return Filter(L, x, y, 0.0f); }
         __device__ WrapFilter wrap(float x, float y) const {
-            if (!wrap_ok(x, y, 0.0f)) return WrapFilter(L, busy, L.grid().min[0], L.grid().min[1], 0.0f);
-            return WrapFilter(L, busy, x, y, 0.0f);
+            if (!wrap_ok(x, y, 0.0f)) return WrapFilter(L, L.grid().min[0], L.grid().min[1], 0.0f);
+            return WrapFilter(L, x, y, 0.0f);
         }
     };
     class Out : public MessageOutBase {
@@ -1276,10 +1277,10 @@ class MessageSpatial3D {
     class In : public SpatialIn<3> {
      public:
         __device__ explicit In(const detail::Launch& l) : SpatialIn<3>(l) {}
-        __device__ Filter operator()(float x, float y, float z) const { return Filter(L, busy, x, y, z); }
+        __device__ Filter operator()(float x, float y, float z) const { return Filter(L, x, y, z); }
         __device__ WrapFilter wrap(float x, float y, float z) const {
-            if (!wrap_ok(x, y, z)) return WrapFilter(L, busy, L.grid().min[0], L.grid().min[1], L.grid().min[2]);
-            return WrapFilter(L, busy, x, y, z);
+            if (!wrap_ok(x, y, z)) return WrapFilter(L, L.grid().min[0], L.grid().min[1], L.grid().min[2]);
+            return WrapFilter(L, x, y, z);
         }
     };
     class Out : public MessageOutBase {

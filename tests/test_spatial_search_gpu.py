@@ -88,3 +88,23 @@ def test_staged_and_unstaged_walks_agree(n, wrap):
         s.close()
     for a, b in zip(*got):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("wrap", [False, True])
+@pytest.mark.parametrize("dims,n", [(2, 1), (2, 700), (3, 1500)])
+def test_searches_of_a_copied_input_list(dims, n, wrap):
+    from flamegpu2_gb300 import sim
+    g = 6
+    pos = np.random.default_rng(n + 1).uniform(0.0, g, (n, dims)).astype(np.float32)
+    counts = np.zeros((g,) * dims, np.int64)
+    np.add.at(counts, _bins(pos, g), 1)
+    around = _neighbourhood_sums(counts, wrap)
+    s = sim.Simulation("spatial_nested", [dims, 0.0, g, 1.0, int(wrap)])
+    s.set_population("agent", n, {k: pos[:, a].copy() for a, k in enumerate(("x", "y", "z")[:dims])})
+    s.step(1)
+    got = _bins(np.stack([s.get("agent", k, np.float32) for k in ("x", "y", "z")[:dims]], 1), g)
+    np.testing.assert_array_equal(s.get("agent", "list_outer", np.uint32), around[got])
+    pairs = _neighbourhood_sums(counts * around, wrap)[got]
+    np.testing.assert_array_equal(s.get("agent", "list_inner", np.uint32), pairs)
+    np.testing.assert_array_equal(s.get("agent", "list_swapped", np.uint32), pairs)
+    s.close()
