@@ -108,3 +108,26 @@ def test_searches_of_a_copied_input_list(dims, n, wrap):
     np.testing.assert_array_equal(s.get("agent", "list_inner", np.uint32), pairs)
     np.testing.assert_array_equal(s.get("agent", "list_swapped", np.uint32), pairs)
     s.close()
+
+
+@pytest.mark.parametrize("wrap", [False, True])
+@pytest.mark.parametrize("g", [1, 2, 3])
+@pytest.mark.parametrize("dims", [2, 3])
+def test_nested_and_copied_searches_on_small_grids(dims, g, wrap):
+    """A grid of one to three bins an axis: the neighbours on both sides of a bin turn round, or are one bin."""
+    from flamegpu2_gb300 import sim
+    n = 90
+    pos = np.random.default_rng(10 * dims + g).uniform(0.0, g, (n, dims)).astype(np.float32)
+    counts = np.zeros((g,) * dims, np.int64)
+    np.add.at(counts, _bins(pos, g), 1)
+    around = _neighbourhood_sums(counts, wrap)
+    s = sim.Simulation("spatial_nested", [dims, 0.0, g, 1.0, int(wrap)])
+    s.set_population("agent", n, {k: pos[:, a].copy() for a, k in enumerate(("x", "y", "z")[:dims])})
+    s.step(1)
+    got = _bins(np.stack([s.get("agent", k, np.float32) for k in ("x", "y", "z")[:dims]], 1), g)
+    pairs = _neighbourhood_sums(counts * around, wrap)[got]
+    for name in ("outer", "copied", "list_outer"):
+        np.testing.assert_array_equal(s.get("agent", name, np.uint32), around[got])
+    for name in ("inner", "list_inner", "list_swapped"):
+        np.testing.assert_array_equal(s.get("agent", name, np.uint32), pairs)
+    s.close()
