@@ -3425,6 +3425,14 @@ void CUDASimulation::setPopulationDevice(const std::string& agent, const std::st
         one_launch = n == 0 || detail::device_range(c.second, static_cast<size_t>(n) * x.elem_bytes[x.ncols], impl->device);
         ++x.ncols;
     }
+    // a variable given twice, or a column of the list itself as another one's
+    // source: copies one after another, each seeing what those before it left
+    for (uint32_t j = 0; one_launch && j < x.ncols; ++j)
+        for (uint32_t k = 0; k < x.ncols; ++k) {
+            const size_t src = static_cast<size_t>(n) * x.elem_bytes[j], dst = static_cast<size_t>(n) * x.elem_bytes[k];
+            const bool meet = x.src[j] < x.dst[k] + dst && x.dst[k] < x.src[j] + src;
+            if (j != k && (x.dst[j] == x.dst[k] || meet)) one_launch = false;
+        }
     // up to 64 MB of aligned device columns: one launch copies them all and
     // sets the count, the next id and the recount, instead of a copy each, two
     // more for the words and a second wait (100,003 Boids 55 us, 31 us so);

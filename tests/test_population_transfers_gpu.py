@@ -101,3 +101,26 @@ def test_columns_copied_to_device_tensors(n):
         np.testing.assert_array_equal(got[offset:offset + m].view(cols[k].dtype), cols[k][:m])
         assert (got[:offset] == -1).all() and (got[offset + m:] == -1).all()
     s.close()
+
+
+@pytest.mark.parametrize("n", [5, 100_003])
+def test_a_variable_given_twice_keeps_its_last_column(n):
+    """The copies go in the order given; the variable that is missing keeps its values."""
+    import ctypes as C
+    import torch
+    from flamegpu2_gb300 import sim
+    s = sim.Simulation("boids_spatial3d")
+    before, after = _columns("Boid", n, 11), _columns("Boid", n, 12)
+    s.set_population("Boid", n, before)
+    names = ["_id", "x", "y", "z", "fx", "fy", "x"]
+    cols = [torch.from_numpy(after[k].view(np.int32)).cuda() for k in names]
+    cols[1].fill_(0)  # the first x
+    torch.cuda.synchronize()
+    rc = sim.core().fgs_reset_population_device(
+        s._h, b"Boid", b"default", n, len(names), (C.c_char_p * len(names))(*[k.encode() for k in names]),
+        (C.c_void_p * len(names))(*[c.data_ptr() for c in cols]), n + 2)
+    assert rc == 0 and s.count("Boid") == n
+    for k in ("x", "y", "z", "fx", "fy"):
+        np.testing.assert_array_equal(s.get("Boid", k, np.float32), after[k])
+    np.testing.assert_array_equal(s.get("Boid", "fz", np.float32), before["fz"])
+    s.close()
