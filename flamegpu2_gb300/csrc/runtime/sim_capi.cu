@@ -109,7 +109,7 @@ extern "C" int fgs_set_population(fgs_sim* s, const char* agent, const char* sta
     return guarded([&] {
         // every variable given: straight to the device, where the transfer
         // also checks that every id is set; a population with ids to assign
-        // goes through AgentVector (the list is left empty by the failed try)
+        // goes through AgentVector
         const auto* ad = s->model->Agent(agent).getData();
         bool all = static_cast<size_t>(nvars) == ad->variables.size();
         std::vector<std::pair<std::string, const void*>> direct;

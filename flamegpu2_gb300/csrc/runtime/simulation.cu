@@ -287,6 +287,7 @@ struct HostXfer {
     uint32_t next_value;
     int32_t id_col;            // set: the id column, checked here (16-byte path only); -1: none
     uint32_t* id_unset;        // set: a host word raised when an id of id_col is unset (0)
+    const uint32_t* refused;   // set: nothing is done where this word is not 0 (k_check_ids); null: none
     const uint32_t* word_src[kHostXferWords];  // get: status words copied to word_dst
     uint32_t* word_dst[kHostXferWords];
     uint32_t nwords;
@@ -302,8 +303,23 @@ __device__ __forceinline__ bool xfer_wide(const HostXfer& x, uint32_t c) {
     return ((reinterpret_cast<uintptr_t>(x.src[c]) | reinterpret_cast<uintptr_t>(x.dst[c])) & 15) == 0;
 }
 
+// Raises *unset (a host word) when one of n ids at a 16-byte boundary is unset (0).
+__global__ void k_check_ids(const uint32_t* ids, uint32_t n, uint32_t* unset) {
+    grid_dependency_enter();
+    const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t bad = 0;
+    for (uint32_t k = tid; k < n / 4u; k += gridDim.x * blockDim.x) {
+        const uint4 v = reinterpret_cast<const uint4*>(ids)[k];
+        bad |= (v.x == 0u) | (v.y == 0u) | (v.z == 0u) | (v.w == 0u);
+    }
+    const uint32_t left = (n & ~3u) + tid;
+    if (left < n) bad |= ids[left] == 0u;
+    if (bad) *unset = 1u;
+}
+
 __global__ void k_host_xfer(const __grid_constant__ HostXfer x) {
     grid_dependency_enter();
+    if (x.refused && *x.refused) return;  // the same in every thread
     const uint32_t rows = x.d_rows ? min(*x.d_rows, x.rows) : x.rows;
     const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
     if (tid == 0) {
@@ -3126,19 +3142,29 @@ void CUDASimulation::setPopulationColumns(const std::string& agent, const std::s
         mapped = x.src[v] != nullptr;
     }
     // the ids: checked (every one set) and their largest found by the transfer
-    // launch when the id column goes in 16-byte pieces, else here on the host
-    const bool dev_ids = mapped && idc < src.size() && n && impl->h_pinned_dev &&
+    // launch when the id column goes in 16-byte pieces, else here on the host.
+    // A refused call leaves the list as it was, but where the column is whole
+    // pieces: there the transfer finds an unset id after it has copied, and the
+    // list is left empty. Ragged columns are checked before: on the host up to
+    // kHostIds ids, above by a launch of their own, which reads them over the
+    // link once more (32,767 ids 5.3 us on the host, 32,769 4.9 us by the
+    // launch; 65,535 10 and 5.9; 999,999 170 and 21)
+    constexpr uint32_t kHostIds = 32768;
+    const bool whole = (static_cast<size_t>(n) * sizeof(id_t)) % 16 == 0;
+    const bool dev_ids = mapped && idc < src.size() && n && impl->h_pinned_dev && (whole || n > kHostIds) &&
                          ((reinterpret_cast<uintptr_t>(x.src[idc]) | reinterpret_cast<uintptr_t>(x.dst[idc])) & 15) == 0;
     id_t mx = 0;
     if (idc < src.size() && n && !dev_ids) {
-        // one branch-free pass (it vectorises): the largest id, and whether any is unset
+        // one pass for the largest id and the smallest (an unset one is 0); as
+        // compares of plain values it vectorises
         const id_t* ids = static_cast<const id_t*>(src[idc]);
-        uint32_t unset = 0;
+        id_t least = ids[0];
         for (uint32_t i = 0; i < n; ++i) {
-            unset |= ids[i] == ID_NOT_SET ? 1u : 0u;
-            mx = std::max(mx, ids[i]);
+            const id_t v = ids[i];
+            least = v < least ? v : least;
+            mx = v > mx ? v : mx;
         }
-        if (unset) THROW exception::InvalidArgument("setPopulationColumns: every _id must be set");
+        if (least == ID_NOT_SET) THROW exception::InvalidArgument("setPopulationColumns: every _id must be set");
     }
     if (mapped) {
         x.ncols = static_cast<uint32_t>(l->cols.size());
@@ -3150,6 +3176,12 @@ void CUDASimulation::setPopulationColumns(const std::string& agent, const std::s
             x.id_col = static_cast<int32_t>(idc);
             impl->h_pinned[4] = 0u;
             x.id_unset = impl->h_pinned_dev + 4;
+            if (!whole) {
+                x.refused = impl->h_pinned_dev + 4;
+                FG_CUDA(detail::launch_kernel(detail::pdl_enabled(), detail::k_check_ids, impl->grid_for(n / 16 + 1, 256, 2),
+                                              256, 0, impl->stream, reinterpret_cast<const uint32_t*>(x.src[idc]), n,
+                                              impl->h_pinned_dev + 4));
+            }
         }
         // the recount of the agents entering the next step, in the same launch
         detail::StepEnd e{};
@@ -3173,9 +3205,13 @@ void CUDASimulation::setPopulationColumns(const std::string& agent, const std::s
     // the recount (done by the transfer launch, else queued behind the
     // copies) before the one wait (the caller's buffers are free again when
     // this returns)
+    if (dev_ids && !whole) {
+        FG_CUDA(cudaStreamSynchronize(impl->stream));
+        if (impl->h_pinned[4] != 0u) THROW exception::InvalidArgument("setPopulationColumns: every _id must be set");
+    }
     l->bound = n;
     impl->forget_counts(mapped);
-    FG_CUDA(cudaStreamSynchronize(impl->stream));
+    if (!dev_ids || whole) FG_CUDA(cudaStreamSynchronize(impl->stream));
     if (dev_ids && impl->h_pinned[4] != 0u) {
         // an unset id: the list is left empty
         FG_CUDA(cudaMemsetAsync(l->d_count, 0, sizeof(uint32_t), impl->stream));
