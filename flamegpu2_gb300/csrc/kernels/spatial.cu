@@ -539,6 +539,10 @@ __device__ __forceinline__ void queue_long_bin(const StabJob& j, uint32_t b, uin
 // place (count of smaller original indices in the bin); long bins are queued
 // as chunks (bucket, chunk index) for k_long. A position's entry is read one
 // round ahead (the first beside the total and the order flag).
+// After a scan whose look-back gave up (FG_ERR_DEVICE_TIMEOUT recorded) bins
+// may overlap, and positions that no row was placed at keep an earlier call's
+// entry, whose row may lie past this call's: here and in the kernels after it
+// an entry is bounded by the last row before it is used as one.
 template <int EMIT>
 __device__ __forceinline__ void stabilize_positions(const StabJob& j, uint32_t blk, uint32_t nblk) {
     const uint32_t stride = nblk * blockDim.x;
@@ -554,7 +558,7 @@ __device__ __forceinline__ void stabilize_positions(const StabJob& j, uint32_t b
     }
     const bool split = EMIT == kEmitPermColumns && j.may_split && rows_in_no_order(j.h, total);
     for (; p < total; p += stride) {
-        const uint32_t i = ahead;
+        const uint32_t i = min(ahead, total - 1u);
         ahead = p + stride < total ? j.perm[p + stride] : 0u;
         const uint32_t b = j.keys[i];
         if (b & kPadBit) {  // padding row of a batch: keeps its slot, carries no message
@@ -562,10 +566,9 @@ __device__ __forceinline__ void stabilize_positions(const StabJob& j, uint32_t b
             continue;
         }
         const uint32_t s = j.pbm[b], e = j.pbm[b + 1];
-        // a PBM from a scan whose look-back gave up (FG_ERR_DEVICE_TIMEOUT
-        // recorded) may run backwards: such a bin is skipped, so no bin is
-        // queued or ranked past the messages (entries never exceed their count)
-        if (e < s) continue;
+        // the PBM of such a scan may run backwards: the bin is skipped, so no
+        // bin is queued or ranked past the rows
+        if (e < s || e > total) continue;
         const uint32_t len = e - s;
         if (len > kShortBin) {
             if (p == s) queue_long_bin(j, b, len);
@@ -687,8 +690,10 @@ __device__ __forceinline__ void long_bins(const StabJob& job, LongSmem& sm, uint
     uint32_t& s_lo = sm.lo;
     uint32_t& s_hi = sm.hi;
     const uint32_t nchunks = min(job.h->long_count, job.chunk_cap);
-    const bool split = EMIT == kEmitPermColumns && job.may_split && nchunks &&
-                       rows_in_no_order(job.h, load_count(job.rows, job.max_n));
+    if (nchunks == 0u) return;  // the same in every thread
+    const uint32_t n = load_count(job.rows, job.max_n);
+    const bool split = EMIT == kEmitPermColumns && job.may_split && rows_in_no_order(job.h, n);
+    auto row = [&](uint32_t p) { return min(perm[p], n - 1u); };  // of a position (see stabilize_positions)
     // warp pass: bins of up to kWarpBin messages
     {
         const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
@@ -701,7 +706,7 @@ __device__ __forceinline__ void long_bins(const StabJob& job, LongSmem& sm, uint
             if (len > kWarpBin || ch.y != 0) continue;  // the same for every lane
             uint32_t lo = 0xFFFFFFFFu, hi = 0u;
             for (uint32_t k = lane; k < len; k += 32u) {
-                const uint32_t i = perm[s + k];
+                const uint32_t i = row(s + k);
                 lo = min(lo, i);
                 hi = max(hi, i);
             }
@@ -714,7 +719,7 @@ __device__ __forceinline__ void long_bins(const StabJob& job, LongSmem& sm, uint
                 for (uint32_t w = lane; w < words; w += 32u) bits[w] = 0u;
                 __syncwarp();
                 for (uint32_t k = lane; k < len; k += 32u) {
-                    const uint32_t d = perm[s + k] - lo;
+                    const uint32_t d = row(s + k) - lo;
                     atomicOr(&bits[d >> 5], 1u << (d & 31u));
                 }
                 __syncwarp();
@@ -741,7 +746,7 @@ __device__ __forceinline__ void long_bins(const StabJob& job, LongSmem& sm, uint
                 }
                 __syncwarp();
                 for (uint32_t k = lane; k < len; k += 32u) {
-                    const uint32_t i = perm[s + k];
+                    const uint32_t i = row(s + k);
                     const uint32_t d = i - lo;
                     emit<EMIT>(rp, sperm, i, s + pre[d >> 5] + __popc(bits[d >> 5] & ((1u << (d & 31u)) - 1u)), split);
                 }
@@ -752,7 +757,7 @@ __device__ __forceinline__ void long_bins(const StabJob& job, LongSmem& sm, uint
                 uint32_t* w = s_idx + wib * kWarpBin;
                 uint32_t p2 = 32;
                 while (p2 < len) p2 <<= 1;
-                for (uint32_t k = lane; k < p2; k += 32u) w[k] = k < len ? perm[s + k] : 0xFFFFFFFFu;
+                for (uint32_t k = lane; k < p2; k += 32u) w[k] = k < len ? row(s + k) : 0xFFFFFFFFu;
                 __syncwarp();
                 for (uint32_t k = 2; k <= p2; k <<= 1) {
                     for (uint32_t j = k >> 1; j > 0; j >>= 1) {
@@ -785,7 +790,7 @@ __device__ __forceinline__ void long_bins(const StabJob& job, LongSmem& sm, uint
             // span of the bin's original indices
             uint32_t lo = 0xFFFFFFFFu, hi = 0u;
             for (uint32_t k = threadIdx.x; k < len; k += blockDim.x) {
-                const uint32_t i = perm[s + k];
+                const uint32_t i = row(s + k);
                 lo = min(lo, i);
                 hi = max(hi, i);
             }
@@ -815,7 +820,7 @@ __device__ __forceinline__ void long_bins(const StabJob& job, LongSmem& sm, uint
                 for (uint32_t w = threadIdx.x; w < words; w += blockDim.x) bits[w] = 0u;
                 __syncthreads();
                 for (uint32_t k = threadIdx.x; k < len; k += blockDim.x) {
-                    const uint32_t d = perm[s + k] - lo;
+                    const uint32_t d = row(s + k) - lo;
                     atomicOr(&bits[d >> 5], 1u << (d & 31u));
                 }
                 __syncthreads();
@@ -833,7 +838,7 @@ __device__ __forceinline__ void long_bins(const StabJob& job, LongSmem& sm, uint
                 }
                 __syncthreads();
                 for (uint32_t k = threadIdx.x; k < len; k += blockDim.x) {
-                    const uint32_t i = perm[s + k];
+                    const uint32_t i = row(s + k);
                     const uint32_t d = i - lo;
                     const uint32_t rank = before[d >> 5] + __popc(bits[d >> 5] & ((1u << (d & 31u)) - 1u));
                     emit<EMIT>(rp, sperm, i, s + rank, split);
@@ -843,7 +848,7 @@ __device__ __forceinline__ void long_bins(const StabJob& job, LongSmem& sm, uint
             uint32_t p2 = 64;
             while (p2 < len) p2 <<= 1;
             __syncthreads();
-            for (uint32_t k = threadIdx.x; k < p2; k += blockDim.x) s_idx[k] = k < len ? perm[s + k] : 0xFFFFFFFFu;
+            for (uint32_t k = threadIdx.x; k < p2; k += blockDim.x) s_idx[k] = k < len ? row(s + k) : 0xFFFFFFFFu;
             __syncthreads();
             for (uint32_t k = 2; k <= p2; k <<= 1) {
                 for (uint32_t j = k >> 1; j > 0; j >>= 1) {
@@ -865,12 +870,12 @@ __device__ __forceinline__ void long_bins(const StabJob& job, LongSmem& sm, uint
         }
         const uint32_t q = s + ch.y * kChunk + threadIdx.x;
         const bool act = q < e;
-        const uint32_t i = act ? perm[q] : 0u;
+        const uint32_t i = act ? row(q) : 0u;
         uint32_t rank = 0;
         for (uint32_t t0 = s; t0 < e; t0 += kRankTile) {
             const uint32_t tn = min(kRankTile, e - t0);
             __syncthreads();
-            for (uint32_t k = threadIdx.x; k < tn; k += blockDim.x) s_idx[k] = perm[t0 + k];
+            for (uint32_t k = threadIdx.x; k < tn; k += blockDim.x) s_idx[k] = row(t0 + k);
             __syncthreads();
             if (act) {
                 uint32_t r = 0;
@@ -915,7 +920,8 @@ __global__ void __launch_bounds__(kThreads) k_long_pair(const __grid_constant__ 
         long_bins<EB>(b, sm, blockIdx.x - ga, gridDim.x - ga);
 }
 
-// Column c moved by the stable permutation, eight rows of a thread in flight.
+// Column c moved by the stable permutation, eight rows of a thread in flight
+// (an entry is bounded by the last row: see stabilize_positions).
 template <typename T>
 __device__ __forceinline__ void gather_column(const fg_column& c, const uint32_t* __restrict__ sperm, uint32_t n) {
     const T* __restrict__ in = static_cast<const T*>(c.in);
@@ -925,7 +931,7 @@ __device__ __forceinline__ void gather_column(const fg_column& c, const uint32_t
         uint32_t i[8];
         T v[8];
 #pragma unroll
-        for (uint32_t m = 0; m < 8; ++m) i[m] = p0 + m * stride < n ? __ldcs(sperm + p0 + m * stride) : 0u;
+        for (uint32_t m = 0; m < 8; ++m) i[m] = p0 + m * stride < n ? min(__ldcs(sperm + p0 + m * stride), n - 1u) : 0u;
 #pragma unroll
         for (uint32_t m = 0; m < 8; ++m)
             if (p0 + m * stride < n) v[m] = in[i[m]];
@@ -949,7 +955,7 @@ __global__ void __launch_bounds__(kThreads) k_gather_columns(const __grid_consta
             gather_column<uint2>(col, sperm, n);
         else
             for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x)
-                copy_column_elem(col, sperm[p], p);
+                copy_column_elem(col, min(sperm[p], n - 1u), p);
     }
 }
 

@@ -127,6 +127,64 @@ def test_compaction_lookback_gives_up_and_recovers(n):
     assert ws.status() == capi.FG_OK
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("crowded", [0, 1])
+@pytest.mark.parametrize("max_n,wide,crowds", [(40_000, 1, 20), (1_700_000, 8, 200)])
+def test_agent_sort_gives_up_and_recovers(max_n, wide, crowds, crowded):
+    """On a workspace whose placement holds rows of an earlier, larger sort; short and long bins; columns moved by the
+    stabilising kernels (40,000 rows) and one after another (more than 96 MB of them)."""
+    import torch
+    capi = _capi()
+    L = capi.lib()
+    st = capi.stream_handle()
+    n = max_n // 2 + 5
+    cells = int(max_n ** 0.5)
+    g = capi.grid(2, (0, 0), (float(cells), float(cells)), 1.0)
+    gen = torch.Generator(device="cuda").manual_seed(max_n)
+    pos = [torch.rand(max_n, device="cuda", generator=gen) * cells for _ in range(2)]
+    if crowded:  # 60% of the rows in a few bins
+        where = torch.randint(0, crowds, (max_n,), device="cuda", generator=gen)
+        some = torch.rand(max_n, device="cuda", generator=gen) < 0.6
+        centre = [torch.randint(0, cells, (crowds,), device="cuda", generator=gen) + 0.5 for _ in range(2)]
+        pos = [torch.where(some, c[where], p).float().contiguous() for c, p in zip(centre, pos)]
+    row = torch.arange(max_n, dtype=torch.int32, device="cuda")
+    ins = pos + [row] + [row.to(torch.int64) + (k << 40) for k in range(wide)]
+    outs = [torch.full_like(c, -1) for c in ins]
+    cols = capi.columns(list(zip(ins, outs)))
+    d_n = torch.tensor([max_n], dtype=torch.int32, device="cuda")
+    ws = capi.Workspace(L.fg_spatial_sort_workspace_size(max_n, g))
+
+    def sort(w):
+        capi.check(L.fg_spatial_sort_agents(g, max_n, d_n.data_ptr(), pos[0].data_ptr(), pos[1].data_ptr(), None, cols,
+                                            len(ins), None, w.ptr, w.nbytes, st), "sort")
+        torch.cuda.synchronize()
+
+    sort(ws)
+    assert ws.status() == capi.FG_OK
+    d_n.fill_(n)
+    for o in outs:
+        o.fill_(-1)
+    ws.set_wait_limit(LIMIT, withhold_first_tile=True)
+    sort(ws)
+    assert ws.status(clear=True) == capi.FG_ERR_DEVICE_TIMEOUT
+    assert int(outs[2].max()) < n  # no row of the earlier sort
+    for o in outs:
+        assert bool((o[n:] == -1).all())
+    ws.set_wait_limit(0, withhold_first_tile=False)
+    fresh = capi.Workspace(L.fg_spatial_sort_workspace_size(max_n, g))
+    sort(fresh)
+    expect = [o.clone() for o in outs]
+    w = torch.full((1,), float(cells), device="cuda")
+    key = (pos[1][:n] / w * w).floor().long() * cells + (pos[0][:n] / w * w).floor().long()
+    assert torch.equal(expect[2][:n].long(), torch.argsort(key, stable=True))
+    for _ in range(2):
+        for o in outs:
+            o.fill_(-1)
+        sort(ws)
+        assert all(torch.equal(a, b) for a, b in zip(outs, expect))
+    assert ws.status() == capi.FG_OK
+
+
 def test_wait_limit_rejects_bad_workspace():
     capi = _capi()
     L = capi.lib()
