@@ -251,7 +251,8 @@ __device__ __forceinline__ void perm_rows(const PermJob& j, uint32_t b, uint32_t
                 record_status(j.h, FG_ERR_WORKSPACE);
         }
         if (j.count_far) {
-            const uint32_t before = __shfl_up_sync(__activemask(), at, 1);
+            const uint32_t left = n - (i - lane_id());  // rows from the warp's first: its lanes still here
+            const uint32_t before = __shfl_up_sync(left < 32u ? (1u << left) - 1u : 0xFFFFFFFFu, at, 1);
             far += (lane_id() > 0u && (at > before ? at - before : before - at) > kFarRows) ? 1u : 0u;
         }
         i = next;
@@ -259,8 +260,8 @@ __device__ __forceinline__ void perm_rows(const PermJob& j, uint32_t b, uint32_t
         slot = ns;
     }
     if (j.count_far) {
-        far = __reduce_add_sync(__activemask(), far);
-        if (far && lane_id() == static_cast<uint32_t>(__ffs(__activemask()) - 1)) atomicAdd(&j.h->far_rows, far);
+        far = __reduce_add_sync(0xFFFFFFFFu, far);
+        if (far && lane_id() == 0u) atomicAdd(&j.h->far_rows, far);
     }
 }
 

@@ -52,3 +52,32 @@ def test_sort_moves_every_column(n, order):
             np.testing.assert_array_equal(o.cpu().numpy(), c[expect])
     np.testing.assert_array_equal(perm.cpu().numpy(), expect)
     assert ws.status() == 0
+
+
+@pytest.mark.parametrize("n", [1, 33, 8_191, 20_000, 100_001, 400_031])
+def test_rows_placed_far_apart_are_counted(n):
+    """What decides how the columns move: rows more than 4,096 places from the row before them in their 32, counted by
+    the placement (the third word of the workspace's header) at ragged ends too. One row a bin, so places are known."""
+    import torch
+    from flamegpu2_gb300 import capi
+    L = capi.lib()
+    room = 1_700_000  # of eight 8-byte columns: more than L2 holds
+    gx, gy = 1024, room // 1024 + 1
+    place = np.random.default_rng(n).permutation(n)
+    x, y = torch.zeros(room, device="cuda"), torch.zeros(room, device="cuda")
+    x[:n] = torch.from_numpy((place % gx + 0.5).astype(np.float32)).cuda()
+    y[:n] = torch.from_numpy((place // gx + 0.5).astype(np.float32)).cuda()
+    wide = [torch.arange(room, device="cuda") + (k << 40) for k in range(8)]
+    outs = [torch.zeros_like(c) for c in wide]
+    g = capi.grid(2, (0, 0), (gx, gy), 1.0)
+    d_n = torch.tensor([n], dtype=torch.int32, device="cuda")
+    ws = capi.Workspace(L.fg_spatial_sort_workspace_size(room, C.byref(g)))
+    capi.check(L.fg_spatial_sort_agents(C.byref(g), room, d_n.data_ptr(), x.data_ptr(), y.data_ptr(), None,
+                                        capi.columns(list(zip(wide, outs))), 8, None, ws.ptr, ws.nbytes,
+                                        capi.stream_handle()), "fg_spatial_sort_agents")
+    torch.cuda.synchronize()
+    far = (np.abs(np.diff(place)) > 4096) & (np.arange(1, n) % 32 != 0)
+    assert int(ws.buf.view(torch.int32)[2]) == far.sum()
+    for k, o in enumerate(outs):
+        np.testing.assert_array_equal(o[:n].cpu().numpy(), np.argsort(place) + (k << 40))
+    assert ws.status() == 0
