@@ -35,6 +35,7 @@
 #include "flamegpu/detail/launch.cuh"
 #include "flamegpu/simulation/CUDASimulation.h"
 #include "flamegpu_gb300/fg_capi.h"
+#include "runtime/device_range.h"
 #include "runtime/internal.h"
 #include "runtime/json.h"
 
@@ -424,34 +425,6 @@ inline void* host_mapped(const void* p) {
         return nullptr;
     }
     return a.type == cudaMemoryTypeHost ? a.devicePointer : nullptr;
-}
-
-// Whether [p, p + bytes) is this device's memory, inside one allocation, on a
-// 16-byte boundary: what a kernel may copy in place of the driver, which looks
-// at the range itself.
-inline bool device_range(const void* p, size_t bytes, int device) {
-    using RangeOf = int (*)(unsigned long long* base, size_t* size, unsigned long long p);  // cuMemGetAddressRange
-    static const RangeOf range_of = [] {
-        void* f = nullptr;
-        cudaDriverEntryPointQueryResult r;
-        if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &f, 12000, cudaEnableDefault, &r) != cudaSuccess) {
-            cudaGetLastError();
-            f = nullptr;
-        }
-        return reinterpret_cast<RangeOf>(f);
-    }();
-    if (!p || !range_of || (reinterpret_cast<uintptr_t>(p) & 15)) return false;
-    cudaPointerAttributes a;
-    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    if (a.type != cudaMemoryTypeDevice || a.device != device) return false;
-    unsigned long long base = 0;
-    size_t size = 0;
-    const unsigned long long at = reinterpret_cast<uintptr_t>(p);
-    if (range_of(&base, &size, at) != 0) return false;
-    return at >= base && at - base <= size && bytes <= size - (at - base);
 }
 
 // A column copied out to the caller's device memory; both on 16 bytes. Copies
