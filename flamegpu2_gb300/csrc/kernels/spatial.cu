@@ -1029,9 +1029,9 @@ uint32_t long_grid_for(uint32_t max_n) {
 }
 
 // Whether a sort's columns may be more than L2 holds (see kFarRows).
-bool splits_columns(const fgk::ColumnParams& cp, uint32_t max_n) {
+bool splits_columns(const fg_column* cols, uint32_t ncols, uint32_t max_n) {
     uint64_t bytes = 0;
-    for (uint32_t c = 0; c < cp.ncols; ++c) bytes += cp.col[c].elem_bytes;
+    for (uint32_t c = 0; c < ncols; ++c) bytes += cols[c].elem_bytes;
     return bytes * max_n > (96ull << 20);
 }
 
@@ -1153,7 +1153,7 @@ int run_pipeline(const fg_spatial_grid* g, const SortGrid& sg, uint32_t nbuckets
     // the scan also compares the keys of rows 32w - 1 and 32w (row order; a batch's keys are never in it)
     const OrderCheck oc{batch.inst ? nullptr : edges, d_n, max_n};
     launch_scan(hist, pbm_out, scan_n, 1, sstat, h, 0, st, key_max, key_floor, oc);
-    const uint32_t may_split = EMIT == kEmitPermColumns && !batch.inst && splits_columns(rp.cp, max_n) ? 1u : 0u;
+    const uint32_t may_split = EMIT == kEmitPermColumns && !batch.inst && splits_columns(rp.cp.col, rp.cp.ncols, max_n) ? 1u : 0u;
     launch(k_perm, grid, kThreads, st, PermJob{max_n, d_n, keys, slot, pbm_out, perm, h, may_split});
     const StabJob sj{rp, keys, pbm_out, perm, sperm, chunks, L.chunk_cap, h, key_max, d_n, max_n, slot, may_split};
     launch(k_stabilize<EMIT>, grid, kThreads, st, sj);
@@ -1220,6 +1220,10 @@ int fgi_spatial_sort_agents(const fg_spatial_grid* g, uint32_t max_n, const uint
         cudaMemcpyAsync(perm_out, sperm, sizeof(uint32_t) * max_n, cudaMemcpyDeviceToDevice, st);
     }
     return check_launch();
+}
+
+uint32_t fgi_spatial_sort_launches(const fg_column* cols, uint32_t ncols, uint32_t max_n, bool keys_ready) {
+    return (keys_ready ? 4u : 5u) + (splits_columns(cols, ncols, max_n) ? 1u : 0u);
 }
 
 // The automatic agent sort of a list and the index build of the spatial

@@ -1683,7 +1683,7 @@ struct SimulationImpl {
                                         static_cast<uint32_t>(cols.size()), nullptr, it->second.first,
                                         it->second.second, stream, f.sort_keyed, stride));
         l.parity ^= 1;
-        kernel_counter += f.sort_keyed ? 4 : 5;
+        kernel_counter += fgi_spatial_sort_launches(cols.data(), static_cast<uint32_t>(cols.size()), l.capacity, f.sort_keyed);
     }
 
     // The record layout of a message list's sorted records: each record word's

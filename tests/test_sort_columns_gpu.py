@@ -81,3 +81,21 @@ def test_rows_placed_far_apart_are_counted(n):
     for k, o in enumerate(outs):
         np.testing.assert_array_equal(o[:n].cpu().numpy(), np.argsort(place) + (k << 40))
     assert ws.status() == 0
+
+
+def test_kernels_of_a_step_count_the_column_gather():
+    """28-byte agents: 96 MB of columns are 3,595,117 agents and a part; above, the sort has one kernel more."""
+    import torch
+    from flamegpu2_gb300 import sim
+    kernels = []
+    for n in (3_595_117, 3_595_118):
+        s = sim.Simulation("spatial_payload", [2, 0.0, 1896.0, 4.0])
+        cols = {k: torch.rand(n, device="cuda") * 1896.0 for k in ("x", "y", "p0", "p1", "p2", "p3")}
+        cols["_id"] = torch.arange(1, n + 1, dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        s.reset_population_device("agent", n, cols, n + 1)
+        s.step(1)
+        s.synchronize()
+        kernels.append(s.stats()["kernels_per_step"])
+        s.close()
+    assert kernels[1] == kernels[0] + 1
