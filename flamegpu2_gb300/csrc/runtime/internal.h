@@ -73,8 +73,15 @@ inline uint32_t index_bits(uint64_t n) {
 // 135 us without, and the predation of 150,000 prey 30.1 and 15.7 us.
 inline bool stage_window_fits(const fg_spatial_grid& g, double per_bin, uint32_t record_words, uint32_t block,
                               unsigned int stage_bytes, uint64_t blocks, uint32_t sms) {
-    // a block's shared memory: the buffer, its header and the searches' range words (228 KB an SM)
-    if (blocks > static_cast<uint64_t>(sms) * ((228u * 1024u) / (stage_bytes + 16u * 1024u))) return false;
+    // a block's shared memory: the buffer, its header and the searches' range
+    // words (228 KB an SM); and registers: staged launches take the variant
+    // without a cap, whose blocks of 128 threads are four an SM at up to 128
+    // registers (the bundled models' take 48 to 96). Small buffers lose nothing
+    // by it: 2D payload agents, one a bin, 24 KB: three blocks an SM 28.3 us a
+    // step unstaged and 27.2 staged, four 29.0 and 28.9, five 31.4 and 31.2,
+    // six and more the same
+    const uint64_t resident = std::min(4u, (228u * 1024u) / (stage_bytes + 16u * 1024u));
+    if (blocks > sms * resident) return false;
     const double span = g.dims == 3 ? static_cast<double>(g.gridDim[0]) * g.gridDim[1] + g.gridDim[0] + 1.0
                                     : static_cast<double>(g.gridDim[0]) + 1.0;
     const double block_bins = std::max(1.0, block / std::max(per_bin, 1e-3));

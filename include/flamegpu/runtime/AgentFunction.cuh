@@ -229,8 +229,7 @@ inline unsigned int device_sm_count() {
 // block: 32, 64 or 128 threads (kAgentBlock divides into whole blocks). A
 // launch of at most one 128-thread block's worth of threads per SM takes the
 // variant compiled without a register cap: its blocks fit the SMs anyway. So
-// does a launch that stages windows: their shared memory holds it to a few
-// blocks per SM.
+// does a launch that stages windows: it has at most four blocks per SM.
 template <typename F>
 cudaError_t launch_agent_function(const LaunchParams& p, unsigned int grid, unsigned int block, unsigned int smem,
                                   cudaStream_t stream, bool pdl) {
