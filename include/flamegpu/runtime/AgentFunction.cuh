@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(kAgentBlock, MINB) agent_function_kernel(const
         if constexpr (STAGE) stage_window<kDims>(L, idx, live != 0xFFFFFFFFu, first);
         first = false;
         if (live == 0xFFFFFFFFu) continue;
-        if (idx < first_row) {  // failed the condition: kept as it is
+        if (!BATCH && idx < first_row) {  // failed the condition: kept as it is
             if (P.death_flags) P.death_flags[idx] = static_cast<uint32_t>(ALIVE);
             ++alive_rows;
             if (P.birth_flags) P.birth_flags[idx] = 0u;
