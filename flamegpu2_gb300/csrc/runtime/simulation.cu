@@ -3442,10 +3442,13 @@ void CUDASimulation::setPopulationDevice(const std::string& agent, const std::st
             const bool meet = x.src[j] < x.dst[k] + dst && x.dst[k] < x.src[j] + src;
             if (j != k && (x.dst[j] == x.dst[k] || meet)) one_launch = false;
         }
-    // up to 64 MB of aligned device columns: one launch copies them all and
+    // up to 64 MiB of aligned device columns: one launch copies them all and
     // sets the count, the next id and the recount, instead of a copy each, two
-    // more for the words and a second wait (100,003 Boids 55 us, 31 us so);
-    // larger populations take the copies, which move more bytes a second
+    // more for the words and a second wait (Boids of 28 bytes: 100,003 20 us a
+    // call and 51 by the copies, 1,000,000 24 and 86, 2,396,000 37 and 99).
+    // Larger populations take the copies; the launch is the faster one there
+    // too (3,000,000 46 and 108, 8,000,000 95 and 150), the line is only as far
+    // as it was first drawn
     if (one_launch && total <= (64u << 20)) {
         x.rows = n;
         x.rows_out = l->d_count;
