@@ -1049,9 +1049,13 @@ class StripCursor {
  * the walk keeps a bit per non-empty bin and reads the next one's bounds ahead,
  * its hash two or three additions from the search's own bin (with the axes'
  * divisions again for every bin, the empty ones too: 200,000 agents at one a
- * bin searched around each neighbour 1,362 us a step, 1,030 so; the
- * 8,388,608-agent Gaussian mixture, wrapped, 440 ms and 419). Its state lies in
- * the listed walk's registers where it can: that walk keeps its speed. */
+ * bin searched around each neighbour 1,360 us a step, 1,142 so; the
+ * 8,388,608-agent Gaussian mixture, wrapped, 440 ms and 425). Its state lies in
+ * the listed walk's registers where it can, and its first look at the bins is a
+ * call: with that look inlined into every search such walks were 10% faster
+ * still (but 8% slower at three agents a bin) and the listed ones up to 0.8%
+ * slower (50,000 to 1,048,576 Boids); with all of it a call on local memory the
+ * listed ones took 1.4 to 2.5 times as long. */
 template <int DIMS>
 class CellCursor {
     static constexpr int kCells = DIMS == 3 ? 27 : 9;
@@ -1059,8 +1063,7 @@ class CellCursor {
     // (MessageSpatial3DDevice.cuh:736-738)
     struct Terms {
         uint32_t hx[3], hy[3], hz[3];
-        __device__ __forceinline__ Terms(const detail::Launch& L, const float (&p)[3]) {
-            const fg_spatial_grid& g = L.grid();
+        __device__ __forceinline__ Terms(const fg_spatial_grid& g, const float (&p)[3]) {
             axis(hx, detail::grid_cell(g, 0, p[0]), g.gridDim[0], 1u);
             axis(hy, detail::grid_cell(g, 1, p[1]), g.gridDim[1], g.gridDim[0]);
             if (DIMS == 3) axis(hz, detail::grid_cell(g, 2, p[2]), g.gridDim[2], g.gridDim[0] * g.gridDim[1]);
@@ -1102,7 +1105,7 @@ class CellCursor {
             : held(L.words_held), owner(!L.words_held) {
             if (!owner) return;
             held = true;
-            const Terms terms(L, p);
+            const Terms terms(L.grid(), p);
             uint32_t* w = column();
             const uint32_t bits = L.P.in_index_bits, base = L.row_base();
             listed = true;
@@ -1131,20 +1134,10 @@ class CellCursor {
             ahead = word();
             return;
         }
-        const Terms terms(L, p);
-        centre = terms.hash(kCells / 2);
-        (DIMS == 3 ? edges : place) = terms.edges() << (DIMS == 3 ? 0 : kCells);
-#pragma unroll 1
-        for (int q = 0; q < 3; ++q) {
-            const uint32_t hx = Terms::pick(terms.hx, q);
-            uint32_t mask = 0;
-#pragma unroll
-            for (int t = 0; t < kCells / 3; ++t) {
-                const uint32_t h = hx + terms.hash_yz(t);
-                mask |= (win.pbm_at(L, h) < win.pbm_at(L, h + 1u) ? 1u : 0u) << t;
-            }
-            place |= mask << (q * (kCells / 3));
-        }
+        const Start start = look(L.grid(), win.gpbm, p[0], p[1], p[2]);
+        centre = start.centre;
+        place = start.place;
+        edges = start.edges;
         read_ahead();
     }
     __device__ __forceinline__ void next(uint32_t& b, uint32_t& e) {
@@ -1162,6 +1155,27 @@ class CellCursor {
     }
 
  private:
+    struct Start {
+        uint32_t centre, place, edges;
+    };
+    // the search's own bin, and the non-empty ones among its neighbours
+    static __device__ __noinline__ Start look(const fg_spatial_grid& g, const uint32_t* pbm, float x, float y, float z) {
+        const float p[3] = {x, y, z};
+        const Terms terms(g, p);
+        Start s{terms.hash(kCells / 2), DIMS == 3 ? 0u : terms.edges() << kCells, DIMS == 3 ? terms.edges() : 0u};
+#pragma unroll 1
+        for (int q = 0; q < 3; ++q) {
+            const uint32_t hx = Terms::pick(terms.hx, q);
+            uint32_t mask = 0;
+#pragma unroll
+            for (int t = 0; t < kCells / 3; ++t) {
+                const uint32_t h = hx + terms.hash_yz(t);
+                mask |= (__ldg(pbm + h) < __ldg(pbm + h + 1u) ? 1u : 0u) << t;
+            }
+            s.place |= mask << (q * (kCells / 3));
+        }
+        return s;
+    }
     __device__ __forceinline__ uint32_t word() const {
         return *static_cast<const uint32_t*>(__cvta_shared_to_generic(place));
     }
