@@ -1049,13 +1049,16 @@ class StripCursor {
  * the walk keeps a bit per non-empty bin and reads the next one's bounds ahead,
  * its hash two or three additions from the search's own bin (with the axes'
  * divisions again for every bin, the empty ones too: 200,000 agents at one a
- * bin searched around each neighbour 1,360 us a step, 1,142 so; the
- * 8,388,608-agent Gaussian mixture, wrapped, 440 ms and 425). Its state lies in
- * the listed walk's registers where it can, and its first look at the bins is a
- * call: with that look inlined into every search such walks were 10% faster
- * still (but 8% slower at three agents a bin) and the listed ones up to 0.8%
- * slower (50,000 to 1,048,576 Boids); with all of it a call on local memory the
- * listed ones took 1.4 to 2.5 times as long. */
+ * bin searched around each neighbour 1,367 us a step, 1,160 so; the
+ * 8,388,608-agent Gaussian mixture, wrapped, 440 ms and 425).
+ * The listed walk keeps its speed: the state of the other one lies in its
+ * registers where it can (a shared address kept as a pointer beside it took
+ * 2,097,152 payload agents at 40 registers from 440 to 490 us; the staged
+ * variant, which has the registers, keeps the pointer: ten steps of 16,384
+ * Boids 304.1 us, 305.4 with the address), and the first look at the bins is a
+ * call, but in a batch (inlined, 1,048,576 Boids 399.5 us instead of 396.7; a
+ * call, 24 batched runs 17.03 ms instead of 16.85). All of it a call on local
+ * memory: the listed walks 1.4 to 2.5 times as long. */
 template <int DIMS>
 class CellCursor {
     static constexpr int kCells = DIMS == 3 ? 27 : 9;
@@ -1130,11 +1133,15 @@ class CellCursor {
         : L(l), win(w), listed(s.listed) {
         if (at_end) return;
         if (listed) {
-            place = static_cast<uint32_t>(__cvta_generic_to_shared(column()));
+            if (L.stage)
+                at = column();
+            else
+                place = static_cast<uint32_t>(__cvta_generic_to_shared(column()));
             ahead = word();
             return;
         }
-        const Start start = look(L.grid(), win.gpbm, p[0], p[1], p[2]);
+        const Start start = L.batch ? look(L.grid(), win.gpbm, p[0], p[1], p[2])
+                                    : look_call(L.grid(), win.gpbm, p[0], p[1], p[2]);
         centre = start.centre;
         place = start.place;
         edges = start.edges;
@@ -1145,7 +1152,10 @@ class CellCursor {
             const uint32_t bits = L.P.in_index_bits;
             b = L.row_base() + (ahead & ((1u << bits) - 1u));
             e = b + (ahead >> bits);
-            place += detail::kAgentBlock * 4u;
+            if (L.stage)
+                at += detail::kAgentBlock;
+            else
+                place += detail::kAgentBlock * 4u;
             ahead = word();  // in flight while this bin is read
             return;
         }
@@ -1159,7 +1169,7 @@ class CellCursor {
         uint32_t centre, place, edges;
     };
     // the search's own bin, and the non-empty ones among its neighbours
-    static __device__ __noinline__ Start look(const fg_spatial_grid& g, const uint32_t* pbm, float x, float y, float z) {
+    static __device__ __forceinline__ Start look(const fg_spatial_grid& g, const uint32_t* pbm, float x, float y, float z) {
         const float p[3] = {x, y, z};
         const Terms terms(g, p);
         Start s{terms.hash(kCells / 2), DIMS == 3 ? 0u : terms.edges() << kCells, DIMS == 3 ? terms.edges() : 0u};
@@ -1176,8 +1186,11 @@ class CellCursor {
         }
         return s;
     }
+    static __device__ __noinline__ Start look_call(const fg_spatial_grid& g, const uint32_t* pbm, float x, float y, float z) {
+        return look(g, pbm, x, y, z);
+    }
     __device__ __forceinline__ uint32_t word() const {
-        return *static_cast<const uint32_t*>(__cvta_shared_to_generic(place));
+        return L.stage ? *at : *static_cast<const uint32_t*>(__cvta_shared_to_generic(place));
     }
     // bin t of the visit order, from the search's own bin: the neighbour on an
     // axis is one cell away, or the axis' length less one at the grid's edge
@@ -1207,6 +1220,7 @@ class CellCursor {
     const detail::Launch L;
     const Window win;
     const bool listed;
+    const uint32_t* at = nullptr;  // listed, staged launches: the word read ahead
     uint32_t place = 0;  // listed: shared address of the word read ahead; else one bit per non-empty bin not yet entered
     uint32_t ahead = 0;  // that word; else the next bin's first message
     // not listed
